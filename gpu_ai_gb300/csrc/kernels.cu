@@ -1,7 +1,8 @@
 // kernels.cu -- playout, move-list and position kernels for sm_103a.
 //
 // Thread-per-playout: each thread keeps its board as four 32-bit words in
-// registers and plays one ply per loop iteration.  The loop is warp-uniform:
+// registers (rotated bitboards seen from the side to move, rot.cuh) and plays
+// one ply per loop iteration.  The loop is warp-uniform:
 // a lane whose game ends writes its int8 outcome and, at the next refill
 // iteration (every fourth), takes the next playout index from a
 // warp-aggregated claim on a global work counter, so the warp never waits for
@@ -10,6 +11,7 @@
 // of a per-thread atomicCAS spin).
 #include "detmath.cuh"
 #include "launch.h"
+#include "rot.cuh"
 #include "rules.cuh"
 
 namespace ga {
@@ -92,27 +94,144 @@ __device__ __forceinline__ void pool_unlock(uint32_t *lock, uint32_t lane) {
 
 __device__ __forceinline__ uint32_t vload(const uint32_t *p) { return *reinterpret_cast<const volatile uint32_t *>(p); }
 
+// The random draws of a game whose ring of eight buffered draws is a column of
+// shared memory: draw k is word k % 8 of the column (consecutive threads,
+// consecutive banks), read with one load where DrawRing selects among eight
+// registers.  refill() keeps at least four draws buffered.
+struct SharedRing {
+  uint32_t *ring;   // word 0 of column 0
+  uint32_t stride;  // columns
+  uint32_t col, k, avail, k0, k1, id0, id1;
+
+  __device__ __forceinline__ void start(uint64_t seed, uint64_t id) {
+    k0 = (uint32_t)seed;
+    k1 = (uint32_t)(seed >> 32);
+    id0 = (uint32_t)id;
+    id1 = (uint32_t)(id >> 32);
+    k = 0;
+    avail = 0;
+  }
+  __device__ __forceinline__ void refill() {
+    if (avail >= 4) return;
+    const uint32_t pos = k + avail;  // multiple of 4
+    uint32_t c[4] = {pos >> 2, id0, id1, 0u};
+    philox4x32_10(c, k0, k1);
+    uint32_t *w = ring + (pos & 4u) * stride + col;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) w[q * stride] = c[q];
+    avail += 4;
+  }
+  __device__ __forceinline__ uint32_t peek() const { return ring[(k & 7u) * stride + col]; }
+  // Move index in [0, n) for n >= 1; a draw is consumed only when n >= 2.
+  __device__ __forceinline__ uint32_t pick(uint32_t n) {
+    const uint32_t i = mulhi_index(peek(), n);  // 0 for n = 1
+    const uint32_t use = n >= 2 ? 1u : 0u;
+    k += use;
+    avail -= use;
+    return i;
+  }
+  __device__ __forceinline__ uint32_t next() {
+    const uint32_t r = peek();
+    k++;
+    avail--;
+    return r;
+  }
+};
+
+// A game as the playout loop holds it: the board and its random draws.  Its
+// words are what moves when a game changes lanes (for a SharedRing the column
+// moves by its number, the draws stay in place).
+struct RotGame {  // uniform random and eps-greedy policies
+  rot::RotBoard b;
+  SharedRing rs;
+  static constexpr int kWords = 8, kCol = 7;  // kCol: the word holding the column
+  // the start position as four words, and a game begun from them
+  __device__ static __forceinline__ uint4 prepare(const Board &at) {
+    const rot::RotBoard r = rot::from_board(Board{at.p1, at.p2, at.kings, at.meta & 0xff01u});
+    return make_uint4(r.own, r.opp, r.kings, r.meta);
+  }
+  __device__ __forceinline__ void start(const uint4 &at, uint64_t seed, uint64_t id) {
+    b = rot::RotBoard{at.x, at.y, at.z, at.w};
+    rs.start(seed, id);
+  }
+  __device__ __forceinline__ bool drawn() const { return b.meta >= ((uint32_t)kDrawPlies << 8); }
+  __device__ __forceinline__ void refill() { rs.refill(); }
+  template <int POLICY>
+  __device__ __forceinline__ int play(bool men_ok, bool king_ok) {
+    if constexpr (POLICY == 2) return rot::play_ply_eps(b, rs, men_ok, king_ok);
+    else return rot::play_ply_random(b, [&](uint32_t n) { return rs.pick(n); }, men_ok, king_ok);
+  }
+  __device__ __forceinline__ void save(uint32_t (&v)[kWords]) const {
+    v[0] = b.own; v[1] = b.opp; v[2] = b.kings; v[3] = b.meta | (rs.avail << 16);
+    v[4] = rs.k; v[5] = rs.id0; v[6] = rs.id1; v[7] = rs.col;
+  }
+  __device__ __forceinline__ void load(const uint32_t (&v)[kWords]) {
+    b.own = v[0]; b.opp = v[1]; b.kings = v[2]; b.meta = v[3] & 0xffffu; rs.avail = v[3] >> 16;
+    rs.k = v[4]; rs.id0 = v[5]; rs.id1 = v[6]; rs.col = v[7];
+  }
+};
+
+struct HeurGame {  // reference heuristic: two draws per move, generated where they are used
+  rot::RotBoard b;
+  rot::BlockDraws rs;
+  static constexpr int kWords = 7, kCol = -1;
+  __device__ static __forceinline__ uint4 prepare(const Board &at) { return RotGame::prepare(at); }
+  __device__ __forceinline__ void start(const uint4 &at, uint64_t seed, uint64_t id) {
+    b = rot::RotBoard{at.x, at.y, at.z, at.w};
+    rs.start(seed, id);
+  }
+  __device__ __forceinline__ bool drawn() const { return b.meta >= ((uint32_t)kDrawPlies << 8); }
+  __device__ __forceinline__ void refill() {}
+  template <int POLICY>
+  __device__ __forceinline__ int play(bool men_ok, bool king_ok) {
+    return rot::play_ply_heuristic(b, rs, men_ok, king_ok,
+                                   [](uint32_t m) { return __reduce_max_sync(__activemask(), m); });
+  }
+  __device__ __forceinline__ void save(uint32_t (&v)[kWords]) const {
+    v[0] = b.own; v[1] = b.opp; v[2] = b.kings; v[3] = b.meta; v[4] = rs.k; v[5] = rs.id0; v[6] = rs.id1;
+  }
+  __device__ __forceinline__ void load(const uint32_t (&v)[kWords]) {
+    b.own = v[0]; b.opp = v[1]; b.kings = v[2]; b.meta = v[3]; rs.k = v[4]; rs.id0 = v[5]; rs.id1 = v[6];
+  }
+};
+
+template <int POLICY> struct GameOf { using type = RotGame; };
+template <> struct GameOf<1> { using type = HeurGame; };
+
+// Bound by the integer (ALU) pipe while every lane has a game (82 % of its
+// peak on 20,011 positions with 4.0 M playouts, 58 % of the lanes active: the
+// rest is the code of the multi-jump plies, which few lanes of a warp run at a
+// time), and by the length of the last games once the work runs out.  Plies on
+// rotated bitboards from the side to move instead of rules.cuh's, draws in
+// shared memory: 372 -> 297 us on the benchmark batch (262,144 playouts), 2.95
+// -> 2.43 ms on the 4.0 M, 1.60 -> 0.86 ms for the reference heuristic's
+// benchmark batch (it no longer walks a cursor per move), 443 -> 368 us for
+// 65,536 eps-greedy playouts through the host call.
 template <int POLICY, int BLOCK, bool POOL>
 __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) playout_kernel(PlayoutArgs a) {
   if (a.dev_sizes != nullptr) {
     a.npos = __ldg(&a.dev_sizes[0]);
     a.total = __ldg(&a.dev_sizes[1]);
   }
+  using Game = typename GameOf<POLICY>::type;
+  constexpr bool kRing = Game::kCol >= 0;  // draws buffered in shared memory
   const uint32_t lane = threadIdx.x & 31u;
-  Board b = {0, 0, 0, 0};
-  uint32_t j = 0, plies_here = 0, game_plies = 0;
+  uint32_t j = 0, plies_here = 0;
   bool have = false, exhausted = false;
 
+  // No ply counter stops a game here: 50 plies without a capture end it, and
+  // a capture takes at least one of at most 64 piece bits off the board.
+  static_assert(64u * kDrawPlies <= kMaxPlies, "the 50-ply rule ends a game within kMaxPlies");
   static_assert(POLICY >= 0 && POLICY <= 2, "policies: 0 random, 1 reference heuristic, 2 eps-greedy");
   {
     // Uniform random policy: at most one draw per ply, so Philox blocks are
-    // generated for the whole warp every fourth iteration (DrawRing keeps four
-    // or more draws buffered) and new games start on those iterations too.
-    // eps-greedy (policy 2, play_ply_eps_sched) takes at most two draws per
-    // ply and refills every second iteration.  The reference heuristic
-    // (policy 1, play_ply_heur_sched) takes two draws per legal move: its ply
-    // loops over the moves for the warp's longest move list and refills the
-    // ring every second step, so Philox still runs for the whole warp at once.
+    // generated for the whole warp every fourth iteration (SharedRing keeps
+    // four or more draws buffered) and new games start on those iterations
+    // too.  eps-greedy (policy 2, rot::play_ply_eps) takes at most two draws
+    // per ply and refills every second iteration.  The reference heuristic
+    // (policy 1, rot::play_ply_heuristic) takes two draws per legal move: its
+    // ply loops over Philox blocks, two moves each, for the warp's longest move
+    // list, so Philox still runs for the whole warp at once.
     // Plies whose capture can be extended take longer code.  Those with one
     // legal move (about two thirds) follow their chain at once; the others,
     // men's multi-jumps (about 1% of plies) and plies where a king's capture
@@ -138,9 +257,12 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
     // Free lanes take ready games before new ones (and pending ones once the
     // work ran out); compaction packs the pools' games too.  A game keeps its
     // whole state (board, stream, ring of draws) wherever it is played, so
-    // the outcomes are the same as without the pools.
-    constexpr int kWords = 17;
+    // the outcomes are the same as without the pools.  Every pool entry owns a
+    // ring column, and a game that moves in or out trades columns with it.
+    constexpr int kWords = Game::kWords + 1;  // ... and the playout index with the pending kind
     constexpr uint32_t kCap = POOL ? kPoolCap : 1u;
+    constexpr uint32_t kColumns = kRing ? BLOCK + (POOL ? 2u * kCap : 0u) : 1u;
+    __shared__ uint32_t s_ring[kRing ? 8u * kColumns : 1u];
     __shared__ uint32_t s_slot[kWords][BLOCK];
     __shared__ uint32_t s_cnt[BLOCK / 32];
     __shared__ uint32_t s_pend[kWords][kCap];   // games waiting for a deferred ply
@@ -148,35 +270,49 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
     __shared__ uint32_t s_pool[4];              // lock, pending games, ready games
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
+    Game g;
+    g.start(make_uint4(0, 0, 0, 0), a.seed, 0);
+    if constexpr (kRing) {
+      g.rs.ring = s_ring;
+      g.rs.stride = kColumns;
+      g.rs.col = threadIdx.x;
+    }
     if constexpr (POOL) {
       if (threadIdx.x < 4) s_pool[threadIdx.x] = 0;
+      if constexpr (kRing) {
+        for (uint32_t q = threadIdx.x; q < kCap; q += BLOCK) {
+          s_pend[Game::kCol][q] = BLOCK + q;
+          s_ready[Game::kCol][q] = BLOCK + kCap + q;
+        }
+      }
       __syncthreads();
     }
-    DrawRing rs;
-    rs.start(0, 0, 0);
     uint32_t pend = 0;    // deferred ply: 0 none, 1 men's multi-jump, 2 king capture search
     bool sparse = false;  // warp-uniform: the work ran out and the warp holds sparse_lanes(POLICY) games or fewer
     constexpr uint32_t kCompactPeriod = compact_period(POLICY);
     constexpr uint32_t kSparseLanes = sparse_lanes(POLICY);
-    auto pick = [&](uint32_t n) { return rs.pick(n); };
-    // a game's state in word q of column idx of a [kWords][stride] area
-    auto put = [&](uint32_t *area, uint32_t stride, uint32_t idx) {
-      const uint32_t v[kWords] = {b.p1, b.p2, b.kings, b.meta, j, game_plies, pend,
-                                  rs.a0, rs.a1, rs.a2, rs.a3, rs.b0, rs.b1, rs.b2, rs.b3, rs.k, rs.avail};
+    // a game's state in word q of column idx of a [kWords][stride] area; with
+    // `trade`, the lane gives its ring column for the entry's
+    auto put = [&](uint32_t *area, uint32_t stride, uint32_t idx, bool trade) {
+      uint32_t v[Game::kWords];
+      g.save(v);
+      if constexpr (kRing) {
+        if (trade) g.rs.col = area[Game::kCol * stride + idx];
+      }
 #pragma unroll
-      for (int q = 0; q < kWords; q++) area[q * stride + idx] = v[q];
+      for (int q = 0; q < Game::kWords; q++) area[q * stride + idx] = v[q];
+      area[Game::kWords * stride + idx] = j | (pend == 2u ? 0x80000000u : 0u);  // a pending men's ply is found again
     };
-    auto take = [&](const uint32_t *area, uint32_t stride, uint32_t idx) {
-      b.p1 = area[idx]; b.p2 = area[stride + idx]; b.kings = area[2 * stride + idx]; b.meta = area[3 * stride + idx];
-      j = area[4 * stride + idx];
-      game_plies = area[5 * stride + idx];
-      pend = area[6 * stride + idx];
-      rs.start(a.seed, stream_of(a, position_of(a, j), j), 0);  // then the buffered draws and counter
-      rs.a0 = area[7 * stride + idx]; rs.a1 = area[8 * stride + idx]; rs.a2 = area[9 * stride + idx];
-      rs.a3 = area[10 * stride + idx]; rs.b0 = area[11 * stride + idx]; rs.b1 = area[12 * stride + idx];
-      rs.b2 = area[13 * stride + idx]; rs.b3 = area[14 * stride + idx];
-      rs.k = area[15 * stride + idx];
-      rs.avail = area[16 * stride + idx];
+    auto take = [&](uint32_t *area, uint32_t stride, uint32_t idx, bool trade) {
+      uint32_t v[Game::kWords];
+#pragma unroll
+      for (int q = 0; q < Game::kWords; q++) v[q] = area[q * stride + idx];
+      if constexpr (kRing) {
+        if (trade) area[Game::kCol * stride + idx] = g.rs.col;
+      }
+      g.load(v);
+      j = area[Game::kWords * stride + idx] & 0x7fffffffu;
+      pend = (area[Game::kWords * stride + idx] >> 31) * 2u;
     };
     // Claim order (equal repetitions, at most BLOCK positions): lanes take
     // the playouts of positions with more pieces first.  Their games are
@@ -219,8 +355,8 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
             const uint32_t npend = vload(&s_pool[1]), nready = vload(&s_pool[2]);
             const uint32_t hm = __ballot_sync(kFull, have);
             if (npend >= 32u && nready + (uint32_t)__popc(hm) <= kCap) {
-              if (have) put(&s_ready[0][0], kCap, nready + __popc(hm & lt));
-              take(&s_pend[0][0], kCap, npend - 32u + lane);
+              if (have) put(&s_ready[0][0], kCap, nready + __popc(hm & lt), true);
+              take(&s_pend[0][0], kCap, npend - 32u + lane, true);
               have = true;
               if (lane == 0) {
                 s_pool[1] = npend - 32u;
@@ -229,7 +365,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
               swapped = true;
             }
             pool_unlock(&s_pool[0], lane);
-            if (swapped) rs.refill();
+            if (swapped) g.refill();
           }
         }
       }
@@ -244,8 +380,8 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
               const uint32_t nr = vload(&s_pool[2]), np = exhausted ? vload(&s_pool[1]) : 0u;
               const uint32_t rank = __popc(fm & lt), k = min((uint32_t)__popc(fm), nr + np);
               if (!have && rank < k) {
-                if (rank < nr) take(&s_ready[0][0], kCap, nr - 1u - rank);
-                else take(&s_pend[0][0], kCap, np - 1u - (rank - nr));
+                if (rank < nr) take(&s_ready[0][0], kCap, nr - 1u - rank, true);
+                else take(&s_pend[0][0], kCap, np - 1u - (rank - nr), true);
                 have = true;
               }
               if (lane == 0) {
@@ -264,11 +400,11 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
             j = (uint32_t)s_order[k] * a.uniform_reps + (j - k * a.uniform_reps);
           }
           const uint32_t p = position_of(a, j);
-          if (GA_IN_BOUNDS(p < a.npos, a.status)) b = load_board(a.pos + p);
-          rs.start(a.seed, stream_of(a, p, j), 0);
-          game_plies = 0;
+          Board at = {0, 0, 0, 0};
+          if (GA_IN_BOUNDS(p < a.npos, a.status)) at = load_board(a.pos + p);
+          g.start(Game::prepare(at), a.seed, stream_of(a, p, j));
         }
-        if (have) rs.refill();
+        if (have) g.refill();
       }
       const bool men_ok = !defer_men(POLICY) || sparse || swapped || (it & (kMenPeriod - 1u)) == kMenPhase;
       const bool king_ok = sparse || swapped || (it & (king_period(POLICY) - 1u)) == kKingPhase;
@@ -276,36 +412,25 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
       do {
         if (!have) break;
         if ((pend == 1u && !men_ok) || (pend == 2u && !king_ok)) break;  // still deferred
-        if (((b.meta >> 8) & 0xffu) >= (uint32_t)kDrawPlies) {
+        if (g.drawn()) {
           if (GA_IN_BOUNDS(j < a.total, a.status)) a.out[j] = 0;
           have = false;
           break;
         }
-        int n;
-        if constexpr (POLICY == 2) {
-          n = play_ply_eps_sched(b, rs, men_ok, king_ok);
-        } else if constexpr (POLICY == 1) {
-          RingOnDemand more{rs};
-          n = play_ply_heur_sched(
-              b, rs, more, men_ok, king_ok, [](uint32_t m) { return __reduce_max_sync(__activemask(), m); },
-              [&] { rs.refill(); });
-        } else {
-          n = play_ply_sched(b, pick, men_ok, king_ok);
-        }
+        const int n = g.template play<POLICY>(men_ok, king_ok);
         if (n == kNeedMen || n == kNeedKing) {
           pend = n == kNeedMen ? 1u : 2u;
           deferred_now = true;
           break;
         }
         pend = 0;
-        if (n > 0 && ++game_plies <= kMaxPlies) {
+        if (n > 0) {
           plies_here++;
           break;
         }
         if (n < 0) atomicOr(a.status, kStatusDepth);
-        else if (n > 0) atomicOr(a.status, kStatusPlyCap);
         if (GA_IN_BOUNDS(j < a.total, a.status))
-          a.out[j] = (int8_t)(n == 0 ? ((b.meta & 1u) ? 1 : -1) : 0);  // side to move cannot move: loses
+          a.out[j] = (int8_t)(n == 0 ? ((g.b.meta & 1u) ? 1 : -1) : 0);  // side to move cannot move: loses
         have = false;
       } while (false);
       if constexpr (POOL) {
@@ -318,7 +443,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
             const uint32_t np = vload(&s_pool[1]);
             const uint32_t k = min((uint32_t)__popc(pm), kCap - np), rank = __popc(pm & lt);
             if (deferred_now && rank < k) {
-              put(&s_pend[0][0], kCap, np + rank);
+              put(&s_pend[0][0], kCap, np + rank, true);
               have = false;
               pend = 0;
             }
@@ -371,7 +496,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
       sparse = __popc(m) <= kSparseLanes;
       if (nr + np == 0 && (total + 31u) / 32u >= busy_warps) continue;  // packing would free no warp
       const uint32_t n_all = min((uint32_t)BLOCK, total + nr + np);  // games the block's lanes hold after packing
-      if (have) put(&s_slot[0][0], BLOCK, before + __popc(m & lt));
+      if (have) put(&s_slot[0][0], BLOCK, before + __popc(m & lt), false);
       if constexpr (POOL) {
         // pool games fill the lanes after the live ones: ready games first
         const uint32_t t = threadIdx.x;
@@ -402,7 +527,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
       }
       have = threadIdx.x < n_all;
       sparse = n_all <= warp * 32u + kSparseLanes;  // this warp now holds min(32, n_all - 32 * warp) games
-      if (have) take(&s_slot[0][0], BLOCK, threadIdx.x);
+      if (have) take(&s_slot[0][0], BLOCK, threadIdx.x, false);
     }
   }
   if (a.plies != nullptr) {

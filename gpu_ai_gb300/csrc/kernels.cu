@@ -44,24 +44,6 @@ __device__ __forceinline__ Board load_board(const Board *p) {
 
 // ---- the playout kernel
 
-// Lanes without a game take the next playout indices: one atomicAdd per warp.
-// Returns true for lanes that got a playout (index in j).
-__device__ __forceinline__ bool claim(const PlayoutArgs &a, bool have, uint32_t &j, bool &exhausted,
-                                      uint32_t lane) {
-  if (exhausted) return false;  // warp-uniform
-  const uint32_t need = __ballot_sync(kFull, !have);
-  if (!need) return false;
-  const uint32_t cnt = __popc(need);
-  const uint32_t leader = __ffs(need) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(a.counter, cnt);
-  base = __shfl_sync(kFull, base, leader);
-  if (base + cnt >= a.total) exhausted = true;
-  if (have) return false;
-  j = base + __popc(need & ((1u << lane) - 1u));
-  return j < a.total;
-}
-
 // Resident blocks per SM that the register budget is sized for: 64 registers
 // a thread for blocks of 256 or more threads (80 for the reference heuristic
 // at 256: 3 blocks), 72 (96 for the reference heuristic) for smaller blocks.
@@ -204,7 +186,7 @@ template <> struct GameOf<1> { using type = HeurGame; };
 // time), and by the length of the last games once the work runs out.  Plies on
 // rotated bitboards from the side to move instead of rules.cuh's, draws in
 // shared memory: 372 -> 297 us on the benchmark batch (262,144 playouts), 2.95
-// -> 2.43 ms on the 4.0 M, 1.60 -> 0.86 ms for the reference heuristic's
+// -> 2.43 ms on the 4.0 M (2.15 ms with claims in bulk), 1.60 -> 0.86 ms for the reference heuristic's
 // benchmark batch (it no longer walks a cursor per move), 443 -> 368 us for
 // 65,536 eps-greedy playouts through the host call.
 template <int POLICY, int BLOCK, bool POOL>
@@ -260,6 +242,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
     // the outcomes are the same as without the pools.  Every pool entry owns a
     // ring column, and a game that moves in or out trades columns with it.
     constexpr int kWords = Game::kWords + 1;  // ... and the playout index with the pending kind
+    static_assert(kWords >= 7, "a stock entry takes seven words");
     constexpr uint32_t kCap = POOL ? kPoolCap : 1u;
     constexpr uint32_t kColumns = kRing ? BLOCK + (POOL ? 2u * kCap : 0u) : 1u;
     __shared__ uint32_t s_ring[kRing ? 8u * kColumns : 1u];
@@ -341,6 +324,21 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
       }
       __syncthreads();
     }
+    // Lanes without a game claim playouts with one atomicAdd per warp.  While
+    // much work remains a warp claims up to 32 at once and keeps them as its
+    // stock: all its lanes look up and convert the positions together (with
+    // uneven repetitions a binary search of the offsets), once per 32 games,
+    // instead of the two or three lanes that need one.  A claim is at most a
+    // quarter of the warp's share of what remains, so a stock is empty again
+    // before the counter runs out; a small batch claims what it needs.  The
+    // stock lives in the warp's part of s_slot, which is free until the block's
+    // stocks are empty (compaction starts after that).
+    // 20,011 positions with 4.0 M uneven playouts: 2.43 -> 2.15 ms; labels of
+    // 16,384 positions by 1,024 playouts each: 7.65 -> 6.47 ms.
+    constexpr uint32_t kBulkClaim = 8;  // the benchmark batch (3 at most) is 1 % slower with bulk claims of any size
+    uint32_t stock = 0, stock_end = 0, chunk = 0;  // games left, entries, next claim: warp-uniform
+    bool dry = false;                              // the counter ran out: warp-uniform
+    const uint32_t chunk_shift = 32u - __clz(gridDim.x * (BLOCK / 32u) * 4u - 1u);
     constexpr uint32_t kRefillMask = POLICY == 2 ? 1u : 3u;
     for (uint32_t it = 0;; ++it) {
       bool swapped = false;  // warp-uniform: this iteration's games came from the pending pool
@@ -393,16 +391,58 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
             }
           }
         }
-        if (claim(a, have, j, exhausted, lane)) {
-          have = true;
-          if (ordered) {  // claim index -> playout index
-            const uint32_t k = j / a.uniform_reps;
-            j = (uint32_t)s_order[k] * a.uniform_reps + (j - k * a.uniform_reps);
+        if (!exhausted) {
+          uint32_t need = __ballot_sync(kFull, !have);
+          if (need && stock == 0 && !dry) {
+            const uint32_t cnt = __popc(need), rank = __popc(need & lt);
+            const bool bulk = chunk >= kBulkClaim;  // warp-uniform
+            const uint32_t m = bulk ? min(32u, chunk) : cnt;
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(a.counter, m);
+            base = __shfl_sync(kFull, base, 0);
+            const uint32_t got = base < a.total ? min(m, a.total - base) : 0u;
+            dry = base + m >= a.total;
+            chunk = dry ? 0u : (a.total - base - m) >> chunk_shift;
+            const uint32_t e = bulk ? lane : rank;
+            if (e < got && (bulk || !have)) {
+              uint32_t q = base + e;
+              if (ordered) {  // claim index -> playout index
+                const uint32_t k = q / a.uniform_reps;
+                q = (uint32_t)s_order[k] * a.uniform_reps + (q - k * a.uniform_reps);
+              }
+              const uint32_t p = position_of(a, q);
+              Board at = {0, 0, 0, 0};
+              if (GA_IN_BOUNDS(p < a.npos, a.status)) at = load_board(a.pos + p);
+              const uint4 v = Game::prepare(at);
+              const uint64_t id = stream_of(a, p, q);
+              if (bulk) {
+                const uint32_t t = warp * 32u + lane;
+                s_slot[0][t] = v.x; s_slot[1][t] = v.y; s_slot[2][t] = v.z; s_slot[3][t] = v.w;
+                s_slot[4][t] = q; s_slot[5][t] = (uint32_t)id; s_slot[6][t] = (uint32_t)(id >> 32);
+              } else {
+                j = q;
+                g.start(v, a.seed, id);
+                have = true;
+              }
+            }
+            stock = bulk ? got : 0u;
+            stock_end = stock;
+            __syncwarp();
           }
-          const uint32_t p = position_of(a, j);
-          Board at = {0, 0, 0, 0};
-          if (GA_IN_BOUNDS(p < a.npos, a.status)) at = load_board(a.pos + p);
-          g.start(Game::prepare(at), a.seed, stream_of(a, p, j));
+          if (need && stock) {  // the warp's stock serves its free lanes
+            need = __ballot_sync(kFull, !have);
+            const uint32_t rank = __popc(need & lt), k = min((uint32_t)__popc(need), stock);
+            if (!have && rank < k) {
+              const uint32_t t = warp * 32u + stock_end - stock + rank;
+              j = s_slot[4][t];
+              g.start(make_uint4(s_slot[0][t], s_slot[1][t], s_slot[2][t], s_slot[3][t]), a.seed,
+                      (uint64_t)s_slot[6][t] << 32 | s_slot[5][t]);
+              have = true;
+            }
+            __syncwarp();
+            stock -= k;
+          }
+          exhausted = dry && stock == 0;
         }
         if (have) g.refill();
       }
@@ -464,13 +504,13 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
       }
       if (!exhausted) {
         // A warp whose lanes are all busy makes no claims: it reads the work
-        // counter itself.  Counter values only grow, and a warp waits at the
+        // counter itself (with games in stock it is not done either way).  Counter values only grow, and a warp waits at the
         // barrier below only after it saw the counter at or past the total, so
         // every other warp of the block sees that too at its next compaction
         // point and joins it: no barrier is needed while work remains.
         uint32_t c = 0;
         if (lane == 0) c = *reinterpret_cast<volatile const uint32_t *>(a.counter);
-        if (__shfl_sync(kFull, c, 0) < a.total) continue;  // warp-uniform
+        if (__shfl_sync(kFull, c, 0) < a.total || stock != 0) continue;  // warp-uniform
         exhausted = true;
       }
       // Only warps that know the work is exhausted get here; they all pass the

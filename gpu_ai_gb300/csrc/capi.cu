@@ -437,7 +437,8 @@ int gpuai_random_positions(gpuai_ctx *ctx, uint64_t seed, uint32_t n, uint32_t m
   cudaStream_t s = ctx->stream;
   const size_t bytes = sizeof(gpuai_board) * (size_t)n;
   CK(ctx->d_aux.reserve(bytes), "device buffer");
-  CK(ga::launch_random_positions(seed, n, min_plies, max_plies, static_cast<ga::Board *>(ctx->d_aux.p), s),
+  CK(ga::launch_random_positions(seed, n, min_plies, max_plies, static_cast<ga::Board *>(ctx->d_aux.p), s,
+                                 ctx->sms),
      "random positions kernel launch");
   CK(cudaMemcpyAsync(out, ctx->d_aux.p, bytes, cudaMemcpyDeviceToHost, s), "D2H boards");
   CK(cudaStreamSynchronize(s), "random positions kernel");
@@ -457,7 +458,7 @@ int gpuai_selfplay_positions(gpuai_ctx *ctx, uint64_t seed, uint32_t n, uint32_t
   int rc = set_device(ctx);
   if (rc) return rc;
   CK(ga::launch_random_positions(seed, n, min_plies, max_plies, reinterpret_cast<ga::Board *>(d_out),
-                                 static_cast<cudaStream_t>(stream), policy),
+                                 static_cast<cudaStream_t>(stream), ctx->sms, policy),
      "self-play positions kernel launch");
   return GPUAI_OK;
 }

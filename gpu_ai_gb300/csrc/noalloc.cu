@@ -144,8 +144,7 @@ extern "C" int gpuai_playouts_noalloc(const gpuai_board *d_pos, const uint32_t *
   a.status = scratch + 1;
   a.plies = reinterpret_cast<unsigned long long *>(scratch + 2);
   const long long resident = (long long)d.sms * d.blocks_per_sm[policy];
-  const long long need = ((long long)total + kBlock[policy] - 1) / kBlock[policy];
-  const int grid = (int)(need < resident ? need : resident);
+  const int grid = (int)((long long)total < resident ? (long long)total : resident);
   e = ga::launch_playouts(a, policy, kBlock[policy], grid, s);
   if (e != cudaSuccess) return cuda_error(e, "playout kernel launch");
   uint32_t status = 0;

@@ -8,14 +8,13 @@
 //
 //   quota_kernel     leaf slots per search this step (min(Q, remaining
 //                    budget)), prefix sums, total leaves / playouts
-//   select_kernel    a warp per search (a block for steps of 128 leaves or
-//                    more): the step's Q leaf slots are split
+//   select_kernel    a block per search: the step's Q leaf slots are split
 //                    over the tree level by level the way the reference's
 //                    GameTree::select splits a batch (src/mcts.cpp:63-157):
 //                    untried children share the slots equally, otherwise in
 //                    proportion to UCB1, remainders to the heaviest children;
-//                    a leaf given more than one slot is expanded; the lanes
-//                    of the warp take one frontier node each
+//                    a leaf given more than one slot is expanded; a group of
+//                    lanes takes a frontier node, a child per lane
 //   playout_kernel   the playout kernel on the leaf boards (sizes and stream
 //                    ids read from device memory)
 //   backprop_kernel  one thread per leaf: visits and score up the path
@@ -29,7 +28,7 @@
 // playout results.
 //
 // The launches of a step are replayed as one CUDA graph.  Because each
-// search is selected by a single warp in a fixed order and its playouts use
+// search is selected by one block in a fixed order and its playouts use
 // its own stream ids, a search's tree and result do not depend on which other
 // searches share the steps.
 //
@@ -54,6 +53,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace ga {
@@ -62,12 +62,10 @@ namespace {
 constexpr uint32_t kExpanded = 1u, kTerminal = 2u, kEvaluated = 4u;  // node state bits (info.y >> 16)
 constexpr int kMaxSelectDepth = 512;
 constexpr uint32_t kStatusSelectDepth = 8u;
-constexpr int kSelectThreads = 128;   // threads per narrow select block: 4 searches of a warp each
-constexpr uint32_t kWideLeaves = 128;  // steps of this many leaves per search or more select with a block per search
-// Team size of a step with Q leaves per search: a warp below kWideLeaves,
-// else a block of 128, 256 or 512 threads (the largest power of two <= Q).
-inline int select_team(uint32_t Q) { return Q < kWideLeaves ? 32 : (Q < 256 ? 128 : (Q < 512 ? 256 : 512)); }
-constexpr uint32_t kMaxLeavesPerStep = 512;  // frontier capacity per search (4 KB of shared memory each)
+// Frontier entries whose expansions take nodes together in a step with Q leaves
+// per search (select_kernel).
+inline uint32_t select_round(uint32_t Q) { return Q < 128 ? 32u : (Q < 256 ? 128u : (Q < 512 ? 256u : 512u)); }
+constexpr uint32_t kMaxLeavesPerStep = 512;  // threads and frontier capacity of the widest select block
 constexpr float kUcbC = 1.41421356f;
 constexpr int kMaxChildren = 64;  // moves per position handled by split_slots
 constexpr uint32_t kUnits = 64;   // learned searches: visit units per leaf slot (score2 = units * (1 + value))
@@ -158,40 +156,59 @@ __global__ void __launch_bounds__(1024) quota_kernel(Table t, uint32_t slots, ui
   }
 }
 
-// Number of children node n would get (its legal moves), 0 for none or when
+// Number of children a node with board b would get (its legal moves), 0 for none or when
 // the game is over (a node's terminal flag is set only for roots; a finished
 // game below the root is found here, when it is first to be expanded).
-__device__ int child_count(const Pool &p, int32_t n) {
-  const uint4 bv = p.board[n];
-  const Board b{bv.x, bv.y, bv.z, bv.w};
+__device__ int child_count(const Board &b) {
   if (((b.meta >> 8) & 0xffu) >= (uint32_t)kDrawPlies) return 0;
   Side sd;
   make_side(b, sd);
-  const int k = count_moves(sd, jumpers(sd));
+  uint32_t M[4];
+  bool capture;
+  const int k = simple_move_masks(sd, M, capture) ? popc(M[0]) + popc(M[1]) + popc(M[2]) + popc(M[3])
+                                                  : count_moves(sd, jumpers(sd));
   return (k > 0 && k <= kMaxChildren) ? k : 0;
 }
 
-// Writes the k children of node n at node indices base.. (called by one lane).
-__device__ void expand_at(const Pool &p, int32_t n, int32_t base, int k) {
-  const uint4 bv = p.board[n];
-  const Board b{bv.x, bv.y, bv.z, bv.w};
+// Writes child c, reached by the move (from, to, removed), of node n.
+__device__ __forceinline__ void write_child(const Pool &p, const Board &b, int32_t n, int32_t c, int from, int to,
+                                            uint32_t removed, int jumps) {
+  Board cb = b;
+  apply_move(cb, from, to, removed);
+  p.board[c] = make_uint4(cb.p1, cb.p2, cb.kings, cb.meta);
+  p.parent[c] = n;
+  p.info[c] = make_uint4(0xffffffffu, 0u, 0u, 0u);
+  p.move[c] = (uint32_t)from | ((uint32_t)to << 8) | ((uint32_t)jumps << 16) |
+              ((promotes(b, from, to) ? 1u : 0u) << 24);
+  p.removed[c] = removed;
+}
+
+// Writes the k children of node n at node indices base.. with G lanes (gl =
+// 0..G-1), a child each: where no capture can continue a lane takes its move
+// straight from the move masks, else it walks the list and writes its share.
+// (The node's own record is its thread's to update.)
+template <uint32_t G>
+__device__ __forceinline__ void expand_group(const Pool &p, const Board &b, int32_t n, int32_t base, int k,
+                                             uint32_t gl) {
   Side sd;
   make_side(b, sd);
-  int32_t c = base;
-  for_each_move(sd, jumpers(sd), [&](int from, int to, uint32_t removed, int jumps, uint32_t) {
-    Board cb = b;
-    apply_move(cb, from, to, removed);
-    p.board[c] = make_uint4(cb.p1, cb.p2, cb.kings, cb.meta);
-    p.parent[c] = n;
-    p.info[c] = make_uint4(0xffffffffu, 0u, 0u, 0u);
-    p.move[c] = (uint32_t)from | ((uint32_t)to << 8) | ((uint32_t)jumps << 16) |
-                ((promotes(b, from, to) ? 1u : 0u) << 24);
-    p.removed[c] = removed;
-    c++;
-    return false;
-  });
-  const uint4 inf = p.info[n];
-  p.info[n] = make_uint4((uint32_t)base, (uint32_t)k | (((inf.y >> 16) | kExpanded) << 16), inf.z, inf.w);
+  uint32_t M[4];
+  bool capture;
+  if (simple_move_masks(sd, M, capture)) {
+    for (int c = (int)gl; c < k; c += (int)G) {
+      int from, to;
+      uint32_t removed;
+      nth_move(M[0], M[1], M[2], M[3], (uint32_t)c, capture, sd.own & ~sd.ownK, from, to, removed);
+      write_child(p, b, n, base + c, from, to, removed, capture ? 1 : 0);
+    }
+  } else {
+    int c = 0;
+    for_each_move(sd, jumpers(sd), [&](int from, int to, uint32_t removed, int jumps, uint32_t) {
+      if ((uint32_t)c % G == gl) write_child(p, b, n, base + c, from, to, removed, jumps);
+      c++;
+      return false;
+    });
+  }
 }
 
 // Splits T slots over the children of node n (the reference's rule,
@@ -206,43 +223,106 @@ __device__ __forceinline__ float ucb_weight(uint4 ci, float lnN) {
   return dm::add(mean, dm::mul(kUcbC, dm::sqrt_(dm::div(lnN, (float)ci.z))));
 }
 
-__device__ int split_slots(const Pool &p, int32_t first, int k, uint32_t parent_visits, uint32_t T,
-                           uint32_t *give) {
+// The children of a node on a group of G lanes, child c on lane c % G as its
+// (c / G)-th of J: what a split reads of them, and the slots it
+// gives.  The k children of a node just expanded (fresh) are not read: none has
+// been visited.
+template <int J, uint32_t G>
+struct Children {
+  static constexpr int kPerLane = J;
+  uint32_t link[J], state[J], visits[J], score2[J], give[J];
+  float prior[J];
+  __device__ __forceinline__ void load(const Pool &p, int32_t first, int k, bool fresh, uint32_t gl,
+                                       const __half *priors) {
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      const int c = (int)gl + (int)G * j;
+      uint4 v = make_uint4(0xffffffffu, 0u, 0u, 0u);
+      __half h = __float2half(0.0f);
+      if (c < k && !fresh) v = p.info[first + c];
+      if (c < k && priors) h = priors[c];
+      link[j] = v.x;
+      state[j] = v.y;
+      visits[j] = v.z;
+      score2[j] = v.w;
+      prior[j] = __half2float(h);
+      give[j] = 0;
+    }
+  }
+  // The children given slots, in child order, to entries at.. of the level's slots.
+  __device__ __forceinline__ void put(int32_t first, int32_t *t_node, uint32_t *t_cnt, uint4 *t_info, uint32_t at,
+                                      uint32_t gl, uint32_t group) const {
+    const uint32_t lower = group & ((1u << (threadIdx.x & 31u)) - 1u);
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      const uint32_t got = __ballot_sync(group, give[j] != 0) & group;
+      if (give[j]) {
+        const uint32_t w = at + __popc(got & lower);
+        t_node[w] = first + (int32_t)(gl + G * j);
+        t_cnt[w] = give[j];
+        t_info[w] = make_uint4(link[j], state[j], visits[j], score2[j]);
+      }
+      at += __popc(got);
+    }
+  }
+};
+
+// Splits T slots over the k children of a node; `lane0` is the group's first
+// lane of the warp.
+template <int J, uint32_t G>
+__device__ __forceinline__ void split_slots(Children<J, G> &ch, int k, uint32_t parent_visits, uint32_t T, uint32_t gl,
+                                            uint32_t lane0, uint32_t group) {
   const float lnN = dm::det_log((float)(parent_visits > 0 ? parent_visits : 1u));
-  float wsum = 0.0f;
-  int untried = 0;
-  for (int c = 0; c < k; c++) {
-    const uint4 ci = p.info[first + c];
-    if (ci.z == 0) untried++;
-    else wsum = dm::add(wsum, ucb_weight(ci, lnN));
+  float w[J], wsum = 0.0f;
+  uint32_t untried = 0;
+#pragma unroll
+  for (int j = 0; j < J; j++) {
+    const bool child = (int)(gl + G * j) < k, fresh = child && ch.visits[j] == 0;
+    w[j] = fresh ? 3.0e38f : -2.0f;  // no child: below every weight
+    if (child && !fresh) w[j] = ucb_weight(make_uint4(0u, 0u, ch.visits[j], ch.score2[j]), lnN);
+    untried += __popc(__ballot_sync(group, fresh) & group);
+  }
+  if (untried == 0) {  // the sum in child order
+#pragma unroll
+    for (int j = 0; j < J; j++)
+#pragma unroll
+      for (uint32_t c = 0; c < G; c++) {
+        const float x = __shfl_sync(group, w[j], lane0 + c);
+        if ((int)(c + G * j) < k) wsum = dm::add(wsum, x);
+      }
   }
   const bool equal = untried == 0 && !(wsum > 0.0f);
+  const float whole = equal ? (float)k : wsum;
+  const uint32_t each = untried ? T / untried : 0u;
   uint32_t assigned = 0;
-  float w[kMaxChildren];
-  for (int c = 0; c < k; c++) {
-    const uint4 ci = p.info[first + c];
-    w[c] = ci.z == 0 ? 3.0e38f : (equal ? 1.0f : ucb_weight(ci, lnN));
-    if (untried > 0) give[c] = ci.z == 0 ? T / (uint32_t)untried : 0u;
-    else give[c] = (uint32_t)dm::mul((float)T, dm::div(w[c], equal ? (float)k : wsum));
-    assigned += give[c];
+#pragma unroll
+  for (int j = 0; j < J; j++) {
+    const bool child = (int)(gl + G * j) < k;
+    if (equal && child) w[j] = 1.0f;
+    if (child) {
+      if (untried) ch.give[j] = ch.visits[j] == 0 ? each : 0u;
+      else ch.give[j] = (uint32_t)dm::mul((float)T, dm::div(w[j], whole));
+    }
+    assigned += ch.give[j];
   }
-  uint64_t extra = 0;  // children that already took one of the remaining slots
-  while (assigned < T) {
-    float mw = -1.0f;
-    int opt = -1;
-    for (int c = 0; c < k; c++)
-      if (!((extra >> c) & 1ull) && w[c] > mw) {
-        mw = w[c];
-        opt = c;
+  assigned = __reduce_add_sync(group, assigned);
+  if (assigned < T) {  // the remainder (fewer than k), one each to the heaviest, first on ties
+    uint32_t heavier[J];
+#pragma unroll
+    for (int j = 0; j < J; j++) heavier[j] = 0;
+#pragma unroll
+    for (int i = 0; i < J; i++)
+#pragma unroll
+      for (uint32_t c = 0; c < G; c++) {
+        const float x = __shfl_sync(group, w[i], lane0 + c);
+#pragma unroll
+        for (int j = 0; j < J; j++)
+          heavier[j] += x > w[j] || (x == w[j] && c + G * i < gl + G * j) ? 1u : 0u;
       }
-    if (opt < 0) break;  // cannot happen: fewer than k slots remain
-    extra |= 1ull << opt;
-    give[opt]++;
-    assigned++;
+#pragma unroll
+    for (int j = 0; j < J; j++)
+      if ((int)(gl + G * j) < k && heavier[j] < T - assigned) ch.give[j]++;
   }
-  int kids = 0;
-  for (int c = 0; c < k; c++) kids += give[c] != 0;
-  return kids;
 }
 
 // Learned searches: splits T slots over the k children of node n one slot at
@@ -251,72 +331,113 @@ __device__ int split_slots(const Pool &p, int32_t first, int k, uint32_t parent_
 // score for the player to move at n (an unvisited child: n's own Q minus
 // kFpuReduction), P its prior (uniform when n has more than kPriors moves or
 // has not been evaluated), N = n's visits and n the child's, in leaf slots.
-// Fills give[0..k) and returns the number of children given slots.
-__device__ int split_puct(const Pool &p, int32_t n, int32_t first, int k, uint32_t parent_visits,
-                          uint32_t parent_score2, uint32_t st, uint32_t T, float c_puct, uint32_t *give) {
-  float q[kMaxChildren], u[kMaxChildren], pr[kMaxChildren], nv[kMaxChildren];
-  const bool priors = (st & kEvaluated) && k <= (int)kPriors;
+// A warp takes a node, a child per lane (two for more than 32).  A slot is a
+// chain of a few operations: the square roots of 32 slots are taken at once, a
+// lane each, a child's next exploration term is ready before the child is
+// chosen, and the scores (never negative) are compared as whole numbers by one
+// reduction.
+template <int J>
+__device__ __forceinline__ void split_puct(Children<J, 32> &ch, int k, bool priors, uint32_t parent_visits,
+                                           uint32_t parent_score2, uint32_t T, float c_puct, uint32_t lane) {
+  constexpr uint32_t kFull = 0xffffffffu;
+  if (k == 1) {
+    if (lane == 0) ch.give[0] = T;
+    return;
+  }
+  float q[J], u[J], un[J], pr[J], nv[J];
   const float fpu =
       parent_visits
           ? fmaxf(0.0f, dm::sub(dm::sub(1.0f, dm::div(dm::mul(0.5f, (float)parent_score2), (float)parent_visits)),
                                 kFpuReduction))
           : 0.5f;
   const float uniform = dm::div(1.0f, (float)k);
-  for (int c = 0; c < k; c++) {
-    const uint4 ci = p.info[first + c];
-    q[c] = ci.z ? dm::div(dm::mul(0.5f, (float)ci.w), (float)ci.z) : fpu;
-    nv[c] = dm::add(1.0f, (float)(ci.z / kUnits));
-    pr[c] = dm::mul(c_puct, priors ? __half2float(p.prior[(size_t)n * kPriors + c]) : uniform);
-    u[c] = dm::div(pr[c], nv[c]);  // exploration term without the sqrt(N) factor
-    give[c] = 0;
+#pragma unroll
+  for (int j = 0; j < J; j++) {
+    const int c = (int)lane + 32 * j;
+    q[j] = ch.visits[j] ? dm::div(dm::mul(0.5f, (float)ch.score2[j]), (float)ch.visits[j]) : fpu;
+    nv[j] = dm::add(1.0f, (float)(ch.visits[j] / kUnits));
+    pr[j] = c < k ? dm::mul(c_puct, priors ? ch.prior[j] : uniform) : 0.0f;
+    u[j] = dm::div(pr[j], nv[j]);  // exploration term without the sqrt(N) factor
+    nv[j] = dm::add(nv[j], 1.0f);
+    un[j] = dm::div(pr[j], nv[j]);  // ... after one more slot
   }
   const float N = (float)(parent_visits / kUnits);
+  float roots = 0.0f;
   for (uint32_t t = 0; t < T; t++) {
-    const float sq = dm::sqrt_(dm::add(dm::add(N, (float)t), 1.0f));
-    int best = 0;
-    float bs = -3.0e38f;
-    for (int c = 0; c < k; c++) {
-      const float sc = dm::add(dm::mul(sq, u[c]), q[c]);
-      if (sc > bs) {
-        bs = sc;
-        best = c;
+    if (t % 32u == 0) roots = dm::sqrt_(dm::add(dm::add(N, (float)(t + lane)), 1.0f));
+    const float sq = __shfl_sync(kFull, roots, t % 32u);
+    uint32_t top = 0, best = 0;  // score + 1 (0: no child), child
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      const uint32_t key =
+          (int)lane + 32 * j < k ? __float_as_uint(dm::add(dm::mul(sq, u[j]), q[j])) + 1u : 0u;
+      const uint32_t m = __reduce_max_sync(kFull, key);
+      const uint32_t first = __ffs(__ballot_sync(kFull, key == m)) - 1u + 32u * j;
+      if (m > top) {
+        top = m;
+        best = first;
       }
     }
-    give[best]++;
-    nv[best] = dm::add(nv[best], 1.0f);
-    u[best] = dm::div(pr[best], nv[best]);
+#pragma unroll
+    for (int j = 0; j < J; j++)
+      if (best == lane + 32u * j) {
+        ch.give[j]++;
+        u[j] = un[j];
+        nv[j] = dm::add(nv[j], 1.0f);
+        un[j] = dm::div(pr[j], nv[j]);
+      }
   }
-  int kids = 0;
-  for (int c = 0; c < k; c++) kids += give[c] != 0;
-  return kids;
 }
 
-// A team of TEAM threads per search (a warp, or the whole 128-thread block
-// for wide steps).  The frontier holds (node, slots) pairs; each round the
-// team takes TEAM frontier entries at a time, expands or splits them, and
-// compacts the children it produced into the next frontier and the leaf slots
-// it produced into the search's output range, in entry order.
-template <bool LEARNED, int TEAM>
-__global__ void __launch_bounds__(TEAM == 32 ? kSelectThreads : TEAM)
-    select_kernel(Pool p, Table t, Leaves l, uint32_t slots, uint32_t ppl, Learned lrn, uint32_t *status) {
-  static_assert(TEAM == 32 || TEAM == 128 || TEAM == 256 || TEAM == 512, "a team is a warp or a whole block");
-  constexpr int kTeams = TEAM == 32 ? kSelectThreads / 32 : 1, kWarps = TEAM / 32;
-  __shared__ int32_t f_node[kTeams][2][kMaxLeavesPerStep];
-  __shared__ uint32_t f_cnt[kTeams][2][kMaxLeavesPerStep];
-  __shared__ uint32_t s_scan[kTeams][2][kWarps];
-  const uint32_t lane = threadIdx.x & 31u, tl = threadIdx.x % TEAM, wt = tl >> 5, ti = threadIdx.x / TEAM;
-  const uint32_t s = blockIdx.x * kTeams + ti;
-  if (s >= slots) return;  // uniform over the team
+// A block of T threads per search (T >= the step's leaves per search).  The
+// frontier holds (node, slots) pairs, a thread each; a level expands or splits
+// them, and its leaf slots and the children given slots go, in entry order, to
+// the search's leaf list and the next frontier, with the records the split has
+// read.  The slots of an entry are a range of the level's slots (their prefix
+// sums), which holds the entry's children or leaf slots in between; a
+// compaction over the slots makes the next frontier.
+//
+// What bounds it is the latency of a level, so each level's serial stretches
+// are shared out: a group of lanes (eight, a warp for learned searches) expands
+// or splits a node, a child per lane.  A thread per entry that enumerated,
+// loaded and split one child after the other took, with the rest of the step,
+// 13.5 against 11.5 ms for 32 steps of 64 searches x 512 leaves, and 17.5
+// against 11.3 ms for 48 steps of 200 learned searches x 64 leaves.
+//
+// Node ranges run out by rounds of `round` entries (a warp's below 128 leaves
+// per search, else 128, 256 or 512): an expansion that does not fit what its
+// round's earlier expansions leave plays out instead, and so do the round's
+// later ones; the next round starts from what was used.
+template <bool LEARNED, int T>
+__global__ void __launch_bounds__(T, 1024 / T)
+    select_kernel(Pool p, Table t, Leaves l, uint32_t slots, uint32_t ppl, uint32_t round, Learned lrn,
+                  uint32_t *status) {
+  constexpr int kWarps = T / 32;
+  constexpr uint32_t G = LEARNED ? 32u : 8u;  // lanes that take a node
+  constexpr uint32_t kLeafSlot = 0x80000000u;
+  __shared__ int32_t f_node[T];   // the frontier: node, slots, the node's record
+  __shared__ uint32_t f_cnt[T];
+  __shared__ uint4 f_info[T];
+  __shared__ int32_t t_node[T];   // the level's slots: a child and its slots, or a leaf slot, or nothing
+  __shared__ uint32_t t_cnt[T];
+  __shared__ uint4 t_info[T];
+  __shared__ int32_t s_leaf[T];   // the leaf slots' nodes
+  __shared__ uint4 s_board[T];    // boards of the nodes to expand
+  __shared__ uint32_t s_scan[2][kWarps];
+  // the entries that expand or split, for their groups: first child, children | state << 8 | fresh << 31 (0:
+  // none), first slot
+  __shared__ int32_t s_first[T];
+  __shared__ uint32_t s_k[T], s_at[T];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t gl = tid % G, gi = tid / G, lane0 = lane & ~(G - 1u), group = (0xffffffffu >> (32u - G)) << lane0;
+  const uint32_t s = blockIdx.x;
   const int32_t root = t.root[s];
-  if (root < 0) return;
+  if (root < 0) return;  // uniform over the block
   const uint32_t off = t.quota_off[s], q = t.quota_off[s + 1] - off;
-  if (q == 0) return;
-  auto team_sync = [&]() {
-    if (TEAM == 32) __syncwarp();
-    else __syncthreads();
-  };
-  // inclusive prefix sums of a and b over the team's threads, and their totals
+  if (q == 0 || !GA_IN_BOUNDS(q <= (uint32_t)T, status)) return;
+  // inclusive prefix sums of a and b over the block's threads, and their totals
   auto scan2 = [&](uint32_t &a, uint32_t &b, uint32_t &ta, uint32_t &tb) {
+#pragma unroll
     for (uint32_t o = 1; o < 32; o <<= 1) {
       const uint32_t x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
       if (lane >= o) {
@@ -324,14 +445,9 @@ __global__ void __launch_bounds__(TEAM == 32 ? kSelectThreads : TEAM)
         b += y;
       }
     }
-    if (TEAM == 32) {
-      ta = __shfl_sync(0xffffffffu, a, 31);
-      tb = __shfl_sync(0xffffffffu, b, 31);
-      return;
-    }
     if (lane == 31) {
-      s_scan[ti][0][wt] = a;
-      s_scan[ti][1][wt] = b;
+      s_scan[0][warp] = a;
+      s_scan[1][warp] = b;
     }
     __syncthreads();
     uint32_t pa = 0, pb = 0;
@@ -339,8 +455,8 @@ __global__ void __launch_bounds__(TEAM == 32 ? kSelectThreads : TEAM)
     tb = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; w++) {
-      const uint32_t va = s_scan[ti][0][w], vb = s_scan[ti][1][w];
-      if ((uint32_t)w < wt) {
+      const uint32_t va = s_scan[0][w], vb = s_scan[1][w];
+      if ((uint32_t)w < warp) {
         pa += va;
         pb += vb;
       }
@@ -351,122 +467,156 @@ __global__ void __launch_bounds__(TEAM == 32 ? kSelectThreads : TEAM)
     b += pb;
     __syncthreads();  // s_scan is reused by the next scan
   };
-  auto team_max = [&](uint32_t x) -> uint32_t {
+  auto block_max = [&](uint32_t x) -> uint32_t {
     x = __reduce_max_sync(0xffffffffu, x);
-    if (TEAM == 32) return x;
-    if (lane == 0) s_scan[ti][0][wt] = x;
+    if (lane == 0) s_scan[0][warp] = x;
     __syncthreads();
     uint32_t m = 0;
 #pragma unroll
-    for (int w = 0; w < kWarps; w++) m = max(m, s_scan[ti][0][w]);
+    for (int w = 0; w < kWarps; w++) m = max(m, s_scan[0][w]);
     __syncthreads();
     return m;
   };
-  int cur = 0;
   uint32_t nf = 1, emitted = 0;
   int32_t node_next = t.node_next[s];
   const int32_t node_end = t.node_end[s];
-  if (tl == 0) {
-    f_node[ti][0][0] = root;
-    f_cnt[ti][0][0] = q;
+  t_cnt[tid] = 0;
+  if (tid == 0) {
+    f_node[0] = root;
+    f_cnt[0] = q;
+    f_info[0] = p.info[root];
   }
-  team_sync();
+  __syncthreads();
   for (int depth = 0; nf > 0; depth++) {
     if (depth >= kMaxSelectDepth) {
-      if (tl == 0) atomicOr(status, kStatusSelectDepth);
+      if (tid == 0) atomicOr(status, kStatusSelectDepth);
       break;
     }
-    uint32_t next_n = 0;
-    for (uint32_t base = 0; base < nf; base += TEAM) {
-      const uint32_t e = base + tl;
-      // pass 1: what each thread's entry produces (children entries or leaf slots)
-      int32_t n = -1, first = 0, k = 0;
-      uint32_t T = 0, leaf = 0, kids = 0, visits = 0, score2 = 0, st = 0;
-      int grow = 0;  // children this thread's node gets if it is expanded now
-      if (e < nf) {
-        n = f_node[ti][cur][e];
-        T = f_cnt[ti][cur][e];
-        const uint4 inf = p.info[n];
-        st = inf.y >> 16;
-        visits = inf.z;
-        score2 = inf.w;
-        first = (int32_t)inf.x;
-        k = (int32_t)(inf.y & 0xffffu);
-        if (st & kTerminal) leaf = T;
-        else if (!(st & kExpanded)) {
-          if (LEARNED) {
-            // a node is expanded once the network has evaluated it
-            if (st & kEvaluated) grow = child_count(p, n);
-            if (grow == 0) leaf = T;
-          } else {
-            if (T == 1) leaf = 1;
-            else grow = child_count(p, n);
-            if (T > 1 && grow == 0) leaf = T;
-          }
-        }
-      }
-      // node indices for this round's expansions, in entry order; an
-      // expansion that does not fit the search's node range plays out
-      // instead (fitting is a prefix of the entries: the inclusive sums grow)
-      uint32_t gx = (uint32_t)grow, unused = 0, gtot = 0, utot = 0;
-      scan2(gx, unused, gtot, utot);
-      const bool fits = grow > 0 && node_next + (int32_t)gx <= node_end;
-      const uint32_t fit_end = team_max(fits ? gx : 0u);
-      if (fits && GA_IN_BOUNDS(node_next + (int32_t)gx <= node_end && (uint32_t)node_end <= p.nodes, status)) {
-        first = node_next + (int32_t)gx - grow;
-        k = grow;
-        expand_at(p, n, first, k);
-      } else if (grow > 0) {
-        leaf = T;
-      }
-      node_next += (int32_t)fit_end;
-      uint32_t give[kMaxChildren];  // this thread's split, written to the next frontier in pass 2
-      if (e < nf && !leaf) {
-        if (LEARNED)
-          kids = (uint32_t)split_puct(p, n, first, k, visits, score2, st, T, lrn.c_puct, give);
-        else
-          kids = (uint32_t)split_slots(p, first, k, visits, T, give);
-      }
-      team_sync();
-      // team prefix sums of children entries and leaf slots
-      uint32_t kx = kids, lx = leaf, ktot = 0, ltot = 0;
-      scan2(kx, lx, ktot, ltot);
-      const uint32_t kid_at = next_n + kx - kids, leaf_at = emitted + lx - leaf;
-      next_n += ktot;
-      emitted += ltot;
-      // pass 2: write children entries and leaf slots
-      if (e < nf) {
-        if (leaf) {
+    // what each thread's entry does: leaf slots, an expansion (grow), a split
+    int32_t n = -1, first = 0, k = 0;
+    uint32_t slots_here = 0, visits = 0, score2 = 0, st = 0;
+    int grow = 0;  // children the node gets if it is expanded now
+    bool leaf = false;
+    if (tid < nf) {
+      n = f_node[tid];
+      slots_here = f_cnt[tid];
+      const uint4 inf = f_info[tid];
+      st = inf.y >> 16;
+      visits = inf.z;
+      score2 = inf.w;
+      first = (int32_t)inf.x;
+      k = (int32_t)(inf.y & 0xffffu);
+      if (st & kTerminal) {
+        leaf = true;
+      } else if (!(st & kExpanded)) {
+        // a learned node is expanded once the network has evaluated it, a
+        // plain one when it is given more than one slot
+        if (LEARNED ? (st & kEvaluated) != 0 : slots_here > 1) {
           const uint4 bv = p.board[n];
-          for (uint32_t r = 0; r < leaf; r++) {
-            const uint32_t o = off + leaf_at + r;
-            if (!GA_IN_BOUNDS(o < slots * lrn.max_leaves && leaf_at + r < q, status)) break;
-            l.board[o] = bv;
-            l.node[o] = n;
-            l.search[o] = (int32_t)s;
+          s_board[tid] = bv;
+          grow = child_count(Board{bv.x, bv.y, bv.z, bv.w});
+        }
+        leaf = grow == 0;
+      }
+    }
+    uint32_t sx = slots_here, gx = (uint32_t)grow, stot = 0, gtot = 0;
+    scan2(sx, gx, stot, gtot);
+    const uint32_t at = sx - slots_here;  // the entry's first slot of the level's
+    bool fresh = false;
+    if (gtot != 0) {  // uniform over the block
+      if (node_next + (int64_t)gtot <= node_end) {
+        fresh = grow > 0;
+        first = fresh ? node_next + (int32_t)gx - grow : first;
+        node_next += (int32_t)gtot;
+      } else {
+        s_at[tid] = gx;
+        __syncthreads();
+        for (uint32_t r = 0; r < nf; r += round) {  // fitting is a prefix of a round's entries: its sums grow
+          const uint32_t in_round = gx - (r ? s_at[r - 1u] : 0u);
+          const bool fits = grow > 0 && tid >= r && tid < r + round && node_next + (int64_t)in_round <= node_end;
+          if (fits) {
+            fresh = true;
+            first = node_next + (int32_t)in_round - grow;
           }
-        } else {
-          uint32_t w = kid_at;
-          for (int c = 0; c < k; c++)
-            if (give[c]) {
-              if (!GA_IN_BOUNDS(w < kMaxLeavesPerStep && (uint32_t)(first + c) < p.nodes, status)) break;
-              f_node[ti][cur ^ 1][w] = first + c;
-              f_cnt[ti][cur ^ 1][w] = give[c];
-              w++;
-            }
+          node_next += (int32_t)block_max(fits ? in_round : 0u);
+        }
+        leaf = leaf || (grow > 0 && !fresh);
+      }
+      if (fresh) {
+        k = grow;
+        if (!GA_IN_BOUNDS(first + k <= node_end && (uint32_t)node_end <= p.nodes, status)) {
+          fresh = false;
+          leaf = true;
         }
       }
-      team_sync();
+      if (fresh) p.info[n] = make_uint4((uint32_t)first, (uint32_t)k | ((st | kExpanded) << 16), visits, score2);
     }
-    cur ^= 1;
-    nf = next_n;
+    if (tid < nf && leaf) {
+      for (uint32_t r = 0; r < slots_here; r++) {
+        t_node[at + r] = n;
+        t_cnt[at + r] = kLeafSlot;
+      }
+    }
+    s_first[tid] = first;
+    s_k[tid] = tid < nf && !leaf ? (uint32_t)k | (st << 8) | (fresh ? 0x80000000u : 0u) : 0u;
+    s_at[tid] = at;
+    __syncthreads();
+    for (uint32_t e = gi; e < nf; e += T / G) {  // uniform over the group
+      const uint32_t ke = s_k[e];
+      if (ke == 0) continue;
+      const int32_t ne = f_node[e], fe = s_first[e];
+      const int kk = (int)(ke & 0xffu);
+      const bool fr = (ke & 0x80000000u) != 0;
+      const bool pri = LEARNED && ((ke >> 8) & kEvaluated) && kk <= (int)kPriors;
+      const uint32_t vis = f_info[e].z;
+      auto split = [&](auto &&ch) {
+        constexpr int J = std::remove_reference_t<decltype(ch)>::kPerLane;
+        ch.load(p, fe, kk, fr, gl, pri ? p.prior + (size_t)ne * kPriors : nullptr);
+        if constexpr (LEARNED) split_puct<J>(ch, kk, pri, vis, f_info[e].w, f_cnt[e], lrn.c_puct, lane);
+        else split_slots<J, G>(ch, kk, vis, f_cnt[e], gl, lane0, group);
+        ch.put(fe, t_node, t_cnt, t_info, s_at[e], gl, group);
+      };
+      if (kk <= (int)G) split(Children<1, G>{});
+      else if (kk <= 2 * (int)G) split(Children<2, G>{});
+      else if constexpr (!LEARNED) split(Children<kMaxChildren / (int)G, G>{});
+      if (fr) {
+        const uint4 bv = s_board[e];
+        expand_group<G>(p, Board{bv.x, bv.y, bv.z, bv.w}, ne, fe, kk, gl);
+      }
+    }
+    __syncthreads();
+    // compaction of the level's slots: the next frontier and the leaf slots
+    const uint32_t have = tid < stot ? t_cnt[tid] : 0u;
+    const int32_t node = tid < stot ? t_node[tid] : 0;
+    const bool is_leaf = have == kLeafSlot;
+    uint32_t kx = have != 0 && !is_leaf ? 1u : 0u, lx = is_leaf ? 1u : 0u, ktot = 0, ltot = 0;
+    scan2(kx, lx, ktot, ltot);
+    t_cnt[tid] = 0;
+    if (is_leaf) {
+      if (GA_IN_BOUNDS(emitted + lx <= q && (uint32_t)node < p.nodes, status)) s_leaf[emitted + lx - 1u] = node;
+    } else if (have && GA_IN_BOUNDS((uint32_t)node < p.nodes, status)) {
+      f_node[kx - 1u] = node;
+      f_cnt[kx - 1u] = have;
+      f_info[kx - 1u] = t_info[tid];
+    }
+    nf = ktot;
+    emitted += ltot;
+    __syncthreads();
   }
-  if (tl == 0) t.node_next[s] = node_next;
-  // per-slot random streams, in slot order
+  // the leaf slots, with their random streams in slot order
   const unsigned long long sbase = t.stream_next[s];
-  for (uint32_t i = tl; i < q; i += TEAM) l.stream[off + i] = sbase + (unsigned long long)i * ppl;
-  team_sync();
-  if (tl == 0) t.stream_next[s] = sbase + (unsigned long long)q * ppl;
+  if (tid < emitted && GA_IN_BOUNDS(off + tid < slots * lrn.max_leaves, status)) {
+    const int32_t n = s_leaf[tid];
+    l.board[off + tid] = p.board[n];
+    l.node[off + tid] = n;
+    l.search[off + tid] = (int32_t)s;
+  }
+  if (tid < q) l.stream[off + tid] = sbase + (unsigned long long)tid * ppl;
+  __syncthreads();
+  if (tid == 0) {
+    t.node_next[s] = node_next;
+    t.stream_next[s] = sbase + (unsigned long long)q * ppl;
+  }
 }
 
 // One thread per leaf: outcomes up the path (score in half points for the
@@ -667,30 +817,18 @@ int enqueue_step(gpuai_searches *s, uint32_t q) {
   // until poll reads them
   SCK(cudaMemsetAsync(s->ctl, 0, sizeof(uint32_t), st), "reset work counter");
   quota_kernel<<<1, 1024, 0, st>>>(s->tab, s->slots, q, s->ppl, s->leaves);
-  // narrow steps: a warp per search, four per block; wide steps (>= 128
-  // leaves per search): a block of 128-512 threads per search, as many
-  // frontier entries per round
-  const int team = select_team(q);
-  const uint32_t per_block = team == 32 ? (uint32_t)(kSelectThreads / 32) : 1u;
-  const uint32_t sel_blocks = (s->slots + per_block - 1) / per_block;
-  const int threads = team == 32 ? kSelectThreads : team;
-  auto sel = [&](auto kernel) {
-    kernel<<<sel_blocks, threads, 0, st>>>(s->pool, s->tab, s->leaves, s->slots, s->ppl, s->lrn, s->ctl + 1);
+  // a block per search with a thread per leaf
+  auto sel = [&](auto kernel, uint32_t threads) {
+    kernel<<<s->slots, threads, 0, st>>>(s->pool, s->tab, s->leaves, s->slots, s->ppl, select_round(q), s->lrn,
+                                         s->ctl + 1);
   };
   if (s->net) {
-    switch (team) {
-      case 32: sel(select_kernel<true, 32>); break;
-      case 128: sel(select_kernel<true, 128>); break;
-      case 256: sel(select_kernel<true, 256>); break;
-      default: sel(select_kernel<true, 512>); break;
-    }
+    if (q <= 256) sel(select_kernel<true, 256>, 256);
+    else sel(select_kernel<true, 512>, 512);
   } else {
-    switch (team) {
-      case 32: sel(select_kernel<false, 32>); break;
-      case 128: sel(select_kernel<false, 128>); break;
-      case 256: sel(select_kernel<false, 256>); break;
-      default: sel(select_kernel<false, 512>); break;
-    }
+    if (q <= 128) sel(select_kernel<false, 128>, 128);
+    else if (q <= 256) sel(select_kernel<false, 256>, 256);
+    else sel(select_kernel<false, 512>, 512);
   }
   PlayoutArgs a;
   a.pos = reinterpret_cast<const Board *>(s->leaves.board);

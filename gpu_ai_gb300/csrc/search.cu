@@ -748,6 +748,31 @@ __global__ void init_search_kernel(Pool p, Table t, int32_t slot, int32_t start,
 
 __global__ void remove_search_kernel(Table t, int32_t slot) { t.root[slot] = -1; }
 
+// A search's root and its children, as gpuai_searches_children reports them.
+struct RootReport {
+  uint4 board, info;
+  int32_t nodes_used;
+  uint32_t pad[3];
+  uint2 child[kMaxChildren];  // visits, score2
+};
+
+// Gathers the report into pinned host memory (one block of kMaxChildren
+// threads).  One launch and one wait in place of four copies and two waits, the
+// second pair of which needed the first's result: 47 -> 18 us for Searches.best.
+__global__ void root_report_kernel(Pool p, Table t, int32_t slot, int32_t root, RootReport *out) {
+  const uint4 info = p.info[root];
+  const uint32_t k = ((info.y >> 16) & kExpanded) ? info.y & 0xffffu : 0u, c = threadIdx.x;
+  if (c < k) {
+    const uint4 ci = p.info[info.x + c];
+    out->child[c] = make_uint2(ci.z, ci.w);
+  }
+  if (c == 0) {
+    out->board = p.board[root];
+    out->info = info;
+    out->nodes_used = t.node_next[slot] - root;
+  }
+}
+
 }  // namespace
 }  // namespace ga
 
@@ -764,6 +789,7 @@ struct gpuai_searches {
   Table tab{};
   Leaves leaves{};
   uint32_t *ctl = nullptr;  // counter, status, plies (2 words)
+  RootReport *report = nullptr;  // pinned host memory, written by root_report_kernel
   std::map<uint32_t, uint32_t> free_ranges;  // start -> length
   std::vector<int32_t> start, cap;           // per slot; start -1 = free slot
   cudaGraphExec_t graph = nullptr;
@@ -980,6 +1006,8 @@ int gpuai_searches_create(int device, uint32_t max_searches, uint32_t pool_nodes
   if (e == cudaSuccess) e = dalloc(s, &s->leaves.out, L * playouts_per_leaf);
   if (e == cudaSuccess) e = dalloc(s, &s->leaves.sizes, 2);
   if (e == cudaSuccess) e = dalloc(s, &s->ctl, 4);
+  if (e == cudaSuccess)
+    e = cudaHostAlloc(reinterpret_cast<void **>(&s->report), sizeof(RootReport), cudaHostAllocMapped);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->tab.root, 0xff, S * sizeof(int32_t), s->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->leaves.sizes, 0, 2 * sizeof(uint32_t), s->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->ctl, 0, 4 * sizeof(uint32_t), s->stream);
@@ -999,6 +1027,7 @@ void gpuai_searches_destroy(gpuai_searches *s) {
   if (s->side) cudaStreamSynchronize(s->side);
   if (s->graph) cudaGraphExecDestroy(s->graph);
   for (void *p : s->allocations) cudaFree(p);
+  if (s->report) cudaFreeHost(s->report);
   if (s->fork) cudaEventDestroy(s->fork);
   if (s->join) cudaEventDestroy(s->join);
   if (s->side) cudaStreamDestroy(s->side);
@@ -1182,36 +1211,22 @@ int gpuai_searches_children(gpuai_searches *s, int32_t slot, gpuai_move *moves, 
   if (slot < 0 || (uint32_t)slot >= s->slots || s->start[slot] < 0)
     return err(GPUAI_ERR_INVALID, "gpuai_searches_children: no such search");
   SCK(cudaSetDevice(s->device), "cudaSetDevice");
-  const int32_t r = s->start[slot];
-  int32_t next = 0;
-  uint4 rb, ri;
-  SCK(cudaMemcpyAsync(&ri, s->pool.info + r, 16, cudaMemcpyDeviceToHost, s->stream), "children");
-  SCK(cudaMemcpyAsync(&rb, s->pool.board + r, 16, cudaMemcpyDeviceToHost, s->stream), "children");
-  SCK(cudaMemcpyAsync(&next, s->tab.node_next + slot, 4, cudaMemcpyDeviceToHost, s->stream), "children");
+  root_report_kernel<<<1, kMaxChildren, 0, s->stream>>>(s->pool, s->tab, slot, s->start[slot], s->report);
+  SCK(cudaGetLastError(), "children");
   SCK(cudaStreamSynchronize(s->stream), "children");
-  if (nodes_used) *nodes_used = (uint32_t)(next - r);
-  const int32_t k = ((ri.y >> 16) & kExpanded) ? (int32_t)(ri.y & 0xffffu) : 0;
-  const int32_t first = (int32_t)ri.x;
+  const RootReport &rep = *s->report;
+  if (nodes_used) *nodes_used = (uint32_t)rep.nodes_used;
+  const int32_t k = ((rep.info.y >> 16) & kExpanded) ? (int32_t)(rep.info.y & 0xffffu) : 0;
   *nchildren = (uint32_t)k;
   if (k <= 0) return GPUAI_OK;
-  std::vector<uint4> ci(k);
-  SCK(cudaMemcpyAsync(ci.data(), s->pool.info + first, 16 * k, cudaMemcpyDeviceToHost, s->stream), "children");
-  SCK(cudaStreamSynchronize(s->stream), "children");
-  std::vector<uint32_t> v(k), sc(k);
-  for (int32_t i = 0; i < k; i++) {
-    v[i] = ci[i].z;
-    sc[i] = ci[i].w;
-  }
   // full move records from the root's move list (same order as the children)
   gpuai::State root_state;
-  root_state.b = gpuai_board{rb.x, rb.y, rb.z, rb.w};
-  const std::vector<gpuai::Move> all_moves = root_state.getMoves();
-  std::vector<gpuai_move> all;
-  for (const gpuai::Move &m : all_moves) all.push_back(m.m);
+  root_state.b = gpuai_board{rep.board.x, rep.board.y, rep.board.z, rep.board.w};
+  const std::vector<gpuai::Move> all = moves ? root_state.getMoves() : std::vector<gpuai::Move>();
   for (uint32_t i = 0; i < (uint32_t)k && i < max_children; i++) {
-    if (visits) visits[i] = v[i];
-    if (score2) score2[i] = sc[i];
-    if (moves && i < all.size()) moves[i] = all[i];
+    if (visits) visits[i] = rep.child[i].x;
+    if (score2) score2[i] = rep.child[i].y;
+    if (moves && i < all.size()) moves[i] = all[i].m;
   }
   return GPUAI_OK;
 }

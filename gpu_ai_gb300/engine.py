@@ -97,8 +97,8 @@ def load_library(path: str = LIB_PATH):
     lib.gpuai_searches_remove.argtypes = [ctypes.c_void_p, ctypes.c_int32]
     lib.gpuai_searches_step.argtypes = [ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_int32]
     lib.gpuai_searches_poll.argtypes = [ctypes.c_void_p, _u64p, _u64p, ctypes.c_uint32, _u32p]
-    lib.gpuai_searches_children.argtypes = [ctypes.c_void_p, ctypes.c_int32, _u8p, _u32p, _u32p, ctypes.c_uint32,
-                                            _u32p, _u32p]
+    lib.gpuai_searches_children.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p,
+                                            ctypes.c_void_p, ctypes.c_uint32, _u32p, _u32p]
     _f32p = ctypes.POINTER(ctypes.c_float)
     vp = ctypes.c_void_p
     lib.gpuai_net_create.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64, ctypes.POINTER(vp)]
@@ -340,8 +340,8 @@ class Searches:
         score2 = np.zeros(max_children, np.uint32)
         n = ctypes.c_uint32()
         used = ctypes.c_uint32()
-        _check(self.lib.gpuai_searches_children(self.h, slot, moves.ctypes.data_as(_u8p), visits.ctypes.data_as(_u32p),
-                                                score2.ctypes.data_as(_u32p), max_children, ctypes.byref(n),
+        _check(self.lib.gpuai_searches_children(self.h, slot, moves.ctypes.data, visits.ctypes.data,
+                                                score2.ctypes.data, max_children, ctypes.byref(n),
                                                 ctypes.byref(used)))
         k = min(n.value, max_children)
         return {"moves": moves[:k], "visits": visits[:k], "score2": score2[:k], "nodes": used.value}

@@ -124,8 +124,8 @@ GA_HD void apply(RotBoard &b, uint32_t from, uint32_t to, uint32_t removed) {
   b.own = reverse(opp);
   b.opp = reverse(own);
   b.kings = reverse(kings);
-  const uint32_t flipped = b.meta ^ 1u;
-  b.meta = removed ? flipped & 1u : flipped + 256u;
+  // the turn passes; the plies since a capture (from bit 8 on) restart after one
+  b.meta = (removed ? b.meta & 1u : b.meta + 256u) ^ 1u;
 }
 
 // A position's jump sources by direction, its first jumps by kind of piece, and
@@ -207,31 +207,40 @@ GA_HD Packed pack(const Masks &m) {
 // subtraction compares them with the index left (bytes of 128 + i - prefix).
 GA_HD void nth(const Packed &p, uint32_t i, uint32_t &from, uint32_t &place) {
   constexpr uint32_t kQuarters = kRows01 | kRows45;
-  const bool u1 = i >= p.low;
-  const uint32_t a = u1 ? p.hi_a : p.lo_a, b = u1 ? p.hi_b : p.lo_b;
-  i -= u1 ? p.low : 0u;
-  uint32_t at = u1 ? kOffset + 16u : kOffset;
+  // (conditional assignments, which compile to predicated instructions, where
+  // selects would be: 2.10 -> 2.05 ms on 20,011 positions with 4.0 M playouts)
+  uint32_t a = p.lo_a, b = p.lo_b, at = kOffset, sel = kQuarters;
+  if (i >= p.low) {
+    i -= p.low;
+    a = p.hi_a;
+    b = p.hi_b;
+    at = kOffset + 16u;
+  }
   uint32_t c = (uint32_t)(popc(a & kQuarters) + popc(b & kQuarters));
-  const bool u2 = i >= c;
-  i -= u2 ? c : 0u;
-  at += u2 ? 8u : 0u;
-  const uint32_t sel = u2 ? ~kQuarters : kQuarters;
+  if (i >= c) {
+    i -= c;
+    at += 8u;
+    sel = ~kQuarters;
+  }
   uint32_t z = rotr((a & sel) | (rotl(b, 8) & ~sel), at);
   c = (uint32_t)popc(z & 0x55555555u);
-  const bool u3 = i >= c;
-  i -= u3 ? c : 0u;
-  at += u3 ? 1u : 0u;
-  z = u3 ? rotr(z, 1) : z;
+  if (i >= c) {
+    i -= c;
+    at += 1u;
+    z >>= 1;
+  }
   c = (uint32_t)popc(z & 0x41414141u);
-  const bool u4 = i >= c;
-  i -= u4 ? c : 0u;
-  at += u4 ? 12u : 0u;
-  z = u4 ? rotr(z, 12) : z;
+  if (i >= c) {
+    i -= c;
+    at += 12u;
+    z = rotr(z, 12);
+  }
   c = (uint32_t)popc(z & 0x01010101u);
-  const bool u5 = i >= c;
-  i -= u5 ? c : 0u;
-  at += u5 ? 6u : 0u;
-  z = u5 ? rotr(z, 6) : z;
+  if (i >= c) {
+    i -= c;
+    at += 6u;
+    z = rotr(z, 6);
+  }
   const uint32_t t = i * 0x01010101u + 0x80808080u - (z & 0x01010101u) * 0x01010101u;
   place = (uint32_t)popc(t & 0x00808080u);
   from = rotl(1u, at);

@@ -32,9 +32,9 @@
 //   adam          sums the partials in a fixed order, updates the FP32 master
 //                 parameters, writes the BF16 copies W1..W3 and W2^T, W3^T
 // Every reduction has a fixed order, so a training run is reproducible.
-// The chain features .. F3, loss, B1, B3, B5 runs on the network's stream,
+// The chain features .. F3, loss, B1, B3, B5, Adam runs on the network's stream,
 // each kernel launched while the one before it drains (programmatic
-// dependent launch); B2 and its row sums run on a second stream, B4 and the
+// dependent launch) and set up before it waits for it; B2 and its row sums run on a second stream, B4 and the
 // remaining row sums on a third.  dZ3 and dZ3^T are all zero between steps:
 // the loss writes at most 32 entries of a row and clear_dz3_kernel zeroes
 // them again once B1 and B2 have read them.
@@ -152,6 +152,7 @@ struct GemmArgs {
   uint32_t *status;
   Epi e;
   uint64_t wait_ns;     // limit of every barrier wait (tc::kWaitLimitNs)
+  uint32_t b_early;     // B holds weights, which no kernel of the step writes: load them before the wait
   uint32_t skip_loads;  // self-test of the bounded waits: issue no TMA load, so the MMA warp's wait runs out
 };
 
@@ -323,10 +324,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   float *vpart = reinterpret_cast<float *>(smem + area + kBarBytes);  // [2][128] value-head partial sums
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t row0 = blockIdx.x * kBM;
-  tc::grid_dep_wait();  // the operands come from the kernel before this one
-  tc::grid_dep_trigger();
   uint32_t rows = g.m_rows;
-  if (g.dev_rows) {
+  if (g.dev_rows) {  // (never launched early: the row count comes from the kernel before)
     const uint32_t d = *g.dev_rows;
     rows = d < rows ? d : rows;
     if (row0 >= rows) return;  // uniform over the CTA, before any barrier or TMEM use
@@ -349,6 +348,21 @@ __global__ void __launch_bounds__(kThreads, 2)
   const uint32_t tmem = *tslot;
   const uint32_t nkb = g.kb_per_split, kb0 = blockIdx.z * nkb;
   uint32_t issued = 0;
+  // What this CTA reads and writes from here on may come from or be read by the
+  // kernel before this one; only the weights do not, whose loads into the ring's
+  // first stages need not wait.  With the barriers, tensor memory and maps set up
+  // above, the loss's moves and Adam's state before their waits too: 8 training
+  // steps of 8192 rows 788 -> 759 us.
+  const uint32_t ahead = g.b_early && !g.skip_loads ? (nkb < nst ? nkb : nst) : 0u;
+  if (warp == 0 && lane == 0) {
+    for (uint32_t i = 0; i < ahead; i++) {
+      tc::mbar_arrive_expect_tx(&full[i], stage_bytes);
+      tc::tma_load_2d(smem + i * stage_bytes + kABytes, &tmB, &full[i], (int32_t)((kb0 + i) * kBK),
+                      (int32_t)(blockIdx.y * bn));
+    }
+  }
+  tc::grid_dep_wait();
+  tc::grid_dep_trigger();
 
   if (warp == 0) {
     if (lane == 0 && !g.skip_loads) {  // TMA producer
@@ -359,9 +373,11 @@ __global__ void __launch_bounds__(kThreads, 2)
           break;
         }
         uint8_t *sa = smem + s * stage_bytes;
-        tc::mbar_arrive_expect_tx(&full[s], stage_bytes);
+        if (i >= ahead) {
+          tc::mbar_arrive_expect_tx(&full[s], stage_bytes);
+          tc::tma_load_2d(sa + kABytes, &tmB, &full[s], (int32_t)((kb0 + i) * kBK), (int32_t)(blockIdx.y * bn));
+        }
         tc::tma_load_2d(sa, &tmA, &full[s], (int32_t)((kb0 + i) * kBK), (int32_t)row0);
-        tc::tma_load_2d(sa + kABytes, &tmB, &full[s], (int32_t)((kb0 + i) * kBK), (int32_t)(blockIdx.y * bn));
         issued = i + 1;
       }
     }
@@ -529,10 +545,44 @@ __device__ __forceinline__ uint32_t lane_pair(const Side &sd, uint32_t J, int &k
 __global__ void loss_kernel(const gpuai_board *boards, const float *z, const float *q, uint32_t n, uint32_t rows,
                             float tau, float vcoef, const float *logits, const float *vraw, bf16 *dZ3, bf16 *dZ3t,
                             uint32_t ldt, float *dv, float *rowloss) {
-  tc::grid_dep_wait();  // the logits and the value come from the kernel before this one
-  tc::grid_dep_trigger();
   const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
   constexpr uint32_t kFull = 0xffffffffu;
+  // The moves and their targets come from the batch alone: found before the
+  // wait for the logits and the value (the kernel before this one's).
+  int k = 0;
+  uint32_t pi = 0x10000u + lane;  // distinct placeholder for lanes without a move
+  float zr = 0.0f, tp = 0.0f;     // tp: target of this lane's pair
+  bool leader = false;
+  if (r < n) {
+    const uint4 bv = __ldg(reinterpret_cast<const uint4 *>(boards) + r);
+    const Board b{bv.x, bv.y, bv.z, bv.w};
+    Side sd;
+    make_side(b, sd);
+    pi = lane_pair(sd, jumpers(sd), k, lane, pi);
+    zr = z[r];
+    if (k >= 1 && k <= (int)kMaxMoves) {  // uniform over the warp
+      const bool act = lane < (uint32_t)k;
+      const float qm = act ? q[(size_t)r * kMaxMoves + lane] : -3.0e38f;
+      float qmax = qm;
+      for (int o = 16; o; o >>= 1) qmax = fmaxf(qmax, __shfl_xor_sync(kFull, qmax, o));
+      const float et = act ? expf((qm - qmax) / tau) : 0.0f;
+      float tsum = et;
+      for (int o = 16; o; o >>= 1) tsum += __shfl_xor_sync(kFull, tsum, o);
+      const float t = et / tsum;
+      const uint32_t grp = __match_any_sync(kFull, pi);
+      leader = act && (uint32_t)(__ffs(grp) - 1) == lane;
+      tp = t;
+      if (__any_sync(kFull, (grp & (grp - 1u)) != 0u)) {  // some pair has two moves (king captures)
+        tp = 0.0f;
+        for (int j = 0; j < 32; j++) {  // the sum over the lanes sharing it, in lane order
+          const float tj = __shfl_sync(kFull, t, j);
+          if ((grp >> j) & 1u) tp += tj;
+        }
+      }
+    }
+  }
+  tc::grid_dep_wait();
+  tc::grid_dep_trigger();
   if (r >= rows) return;
   if (r >= n) {
     if (lane == 0) {
@@ -544,38 +594,12 @@ __global__ void loss_kernel(const gpuai_board *boards, const float *z, const flo
   const float inv_n = 1.0f / (float)n;
   if (lane == 0) {
     const float th = tanhf(vraw[r]);
-    const float e = th - z[r];
+    const float e = th - zr;
     dv[r] = vcoef * 2.0f * e * (1.0f - th * th) * inv_n;
     rowloss[2 * r + 1] = e * e;
   }
-  const uint4 bv = __ldg(reinterpret_cast<const uint4 *>(boards) + r);
-  const Board b{bv.x, bv.y, bv.z, bv.w};
-  Side sd;
-  make_side(b, sd);
-  const uint32_t J = jumpers(sd);
-  int k = 0;
-  // distinct placeholder for lanes without a move
-  const uint32_t pi = lane_pair(sd, J, k, lane, 0x10000u + lane);
   float ce = 0.0f;
-  if (k >= 1 && k <= (int)kMaxMoves) {  // uniform over the warp
-    const bool act = lane < (uint32_t)k;
-    const float qm = act ? q[(size_t)r * kMaxMoves + lane] : -3.0e38f;
-    float qmax = qm;
-    for (int o = 16; o; o >>= 1) qmax = fmaxf(qmax, __shfl_xor_sync(kFull, qmax, o));
-    const float et = act ? expf((qm - qmax) / tau) : 0.0f;
-    float tsum = et;
-    for (int o = 16; o; o >>= 1) tsum += __shfl_xor_sync(kFull, tsum, o);
-    const float t = et / tsum;
-    const uint32_t grp = __match_any_sync(kFull, pi);
-    const bool leader = act && (uint32_t)(__ffs(grp) - 1) == lane;
-    float tp = t;  // target of this lane's pair: sum over the lanes sharing it, in lane order
-    if (__any_sync(kFull, (grp & (grp - 1u)) != 0u)) {  // some pair has two moves (king captures)
-      tp = 0.0f;
-      for (int j = 0; j < 32; j++) {
-        const float tj = __shfl_sync(kFull, t, j);
-        if ((grp >> j) & 1u) tp += tj;
-      }
-    }
+  if (k >= 1 && k <= (int)kMaxMoves) {
     const float lg = leader ? logits[(size_t)r * kOut + pi] : -3.0e38f;
     float lmax = lg;
     for (int o = 16; o; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(kFull, lmax, o));
@@ -809,10 +833,15 @@ __device__ __forceinline__ float sum_partials(const float *p, size_t stride, uin
   return g;
 }
 
+// The state is read before the wait for the gradients (in the training step the
+// launch is early, beside dW1's product).
 __global__ void adam_kernel(AdamArgs a) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kParams) return;
-  float w = a.w[i];
+  const bool in = i < kParams;
+  float w = in ? a.w[i] : 0.0f;
+  const float m0 = in && a.mode == 0 ? a.m[i] : 0.0f, v0 = in && a.mode == 0 ? a.v[i] : 0.0f;
+  tc::grid_dep_wait();
+  if (!in) return;
   if (a.mode != 2) {
     float g = 0.0f;
     if (i < oB1) {
@@ -829,8 +858,8 @@ __global__ void adam_kernel(AdamArgs a) {
       return;
     }
     const float lr = a.lr, bc1 = a.bc1, bc2 = a.bc2;
-    const float m = kBeta1 * a.m[i] + (1.0f - kBeta1) * g;
-    const float v = kBeta2 * a.v[i] + (1.0f - kBeta2) * g * g;
+    const float m = kBeta1 * m0 + (1.0f - kBeta1) * g;
+    const float v = kBeta2 * v0 + (1.0f - kBeta2) * g * g;
     a.m[i] = m;
     a.v[i] = v;
     w -= lr * (m / bc1) / (sqrtf(v / bc2) + kAdamEps);
@@ -987,7 +1016,8 @@ cudaError_t launch(void (*kernel)(Params...), dim3 grid, uint32_t threads, uint3
 
 cudaError_t gemm(const CUtensorMap &a, const CUtensorMap &b, uint32_t m_rows, uint32_t n_total, uint32_t bn,
                  uint32_t kb_total, uint32_t splits, const uint32_t *dev_rows, uint32_t *status, const Epi &e,
-                 cudaStream_t s, bool pdl = false, uint64_t wait_ns = tc::kWaitLimitNs, bool skip_loads = false) {
+                 cudaStream_t s, bool pdl = false, bool b_early = false, uint64_t wait_ns = tc::kWaitLimitNs,
+                 bool skip_loads = false) {
   if (m_rows % kBM || bn % 64 || bn == 0 || bn > 256 || n_total % bn || splits == 0 || kb_total % splits)
     return cudaErrorInvalidValue;
   if ((e.flags & kEpiVdot) && !(n_total == 256u && (bn == 128u || bn == 256u)))  // the value head's two tiles
@@ -1011,6 +1041,7 @@ cudaError_t gemm(const CUtensorMap &a, const CUtensorMap &b, uint32_t m_rows, ui
   g.status = status;
   g.e = e;
   g.wait_ns = wait_ns;
+  g.b_early = pdl && b_early ? 1u : 0u;
   g.skip_loads = skip_loads ? 1u : 0u;
   const uint32_t ring = g.stages * stage_bytes;
   const uint32_t smem = (ring > kStageBytes ? ring : kStageBytes) + kSmemExtra;
@@ -1088,7 +1119,7 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   e1.ld_b = kH;
   e1.out_t = net->H1t;
   e1.ld_t = net->rows;
-  if ((e = gemm(w.mX, net->mW1, rows, kH, kBnF1, kInPad / kBK, 1, dev_n, status, e1, s, train)) != cudaSuccess)
+  if ((e = gemm(w.mX, net->mW1, rows, kH, kBnF1, kInPad / kBK, 1, dev_n, status, e1, s, train, true)) != cudaSuccess)
     return e;
   Epi e2 = e1;
   e2.flags |= kEpiVdot;
@@ -1102,7 +1133,7 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   // idle, in 256-column tiles once the row blocks alone fill the SMs
   const bool wide2 = rows / kBM >= sm_count();
   if ((e = gemm(w.mH1, wide2 ? net->mW2w : net->mW2, rows, kH, wide2 ? 2u * kBnF2 : kBnF2, kH / kBK, 1, dev_n, status,
-                e2, s, train)) != cudaSuccess)
+                e2, s, train, true)) != cudaSuccess)
     return e;
   Epi e3;
   e3.flags = kEpiBias | kEpiVsum | (w.logits_b ? kEpiB16 : kEpiF32);
@@ -1115,7 +1146,7 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   e3.ld_f32 = kOut;
   e3.out_b = w.logits_b;
   e3.ld_b = kOut;
-  return gemm(w.mH2, net->mW3, rows, kOut, kBnF3, kH / kBK, 1, dev_n, status, e3, s, train);
+  return gemm(w.mH2, net->mW3, rows, kOut, kBnF3, kH / kBK, 1, dev_n, status, e3, s, train, true);
 }
 
 // Forward + backward on rows [0, n) of the training workspace; gradients are
@@ -1170,7 +1201,7 @@ cudaError_t backward_impl(gpuai_net *net, const gpuai_board *boards, const float
   b1.ld_t = L;
   const bool wide = (B / kBM) * (kH / kBnB1) >= sm_count();  // 128-wide tiles of B1 and B3 fill the SMs
   if ((e = gemm(net->mdZ3, wide ? net->mW3T : net->mW3Tn, B, kH, wide ? kBnB1 : kBnNarrow, kOut / kBK, 1, nullptr,
-                net->status, b1, s, true)) != cudaSuccess)
+                net->status, b1, s, true, true)) != cudaSuccess)
     return e;
   // third stream, after dZ2: dW2 partials and db2; side stream: dZ3 (read
   // by dZ2's product) and dZ3^T (dW3's) back to zero, which nothing in the
@@ -1198,7 +1229,7 @@ cudaError_t backward_impl(gpuai_net *net, const gpuai_board *boards, const float
   b3.out_t = net->dZ1t;
   b3.ld_t = L;
   if ((e = gemm(net->mdZ2, wide ? net->mW2T : net->mW2Tn, B, kH, wide ? kBnB3 : kBnNarrow, kH / kBK, 1, nullptr,
-                net->status, b3, s, true)) != cudaSuccess)
+                net->status, b3, s, true, true)) != cudaSuccess)
     return e;
   // third stream, after dZ1: db1; then the main stream waits for both side streams
   if ((e = cudaEventRecord(net->ev_b3, s)) != cudaSuccess) return e;
@@ -1253,8 +1284,7 @@ cudaError_t run_adam(gpuai_net *net, uint32_t mode, const uint32_t *splits, floa
   a.W3b = net->W3b;
   a.W2T = net->W2T;
   a.W3T = net->W3T;
-  adam_kernel<<<(uint32_t)((kParams + 255) / 256), 256, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch(adam_kernel, dim3((uint32_t)((kParams + 255) / 256)), 256, 0, s, mode == 0, a);
 }
 
 template <class... P>
@@ -1685,7 +1715,7 @@ int gpuai_net_wait_selftest(gpuai_net *net, uint32_t wait_limit_us, uint32_t *st
   e1.bias = net->params + oB1;
   e1.out_b = net->fw.H1;
   e1.ld_b = kH;
-  NCK(gemm(net->fw.mX, net->mW1, kBM, kH, kBnF1, kInPad / kBK, 1, nullptr, net->status, e1, s, false,
+  NCK(gemm(net->fw.mX, net->mW1, kBM, kH, kBnF1, kInPad / kBK, 1, nullptr, net->status, e1, s, false, false,
            (uint64_t)wait_limit_us * 1000u, true),
       "self-test launch");
   uint32_t st = 0;

@@ -185,6 +185,9 @@ struct Packed {
   uint32_t low, n;                  // moves in the low half, in all
 };
 
+// The two quarters (rows 0-1 and 4-5) whose moves come first in their half.
+constexpr uint32_t kQuarters = kRows01 | kRows45;
+
 GA_HD Packed pack(const Masks &m) {
   const uint32_t r2 = rotl(m.m2, 16), r3 = rotl(m.m3, 16);
   Packed p;
@@ -206,7 +209,6 @@ GA_HD Packed pack(const Masks &m) {
 // bit per mask, 8 apart: one multiply takes their prefix sums, one
 // subtraction compares them with the index left (bytes of 128 + i - prefix).
 GA_HD void nth(const Packed &p, uint32_t i, uint32_t &from, uint32_t &place) {
-  constexpr uint32_t kQuarters = kRows01 | kRows45;
   // (conditional assignments, which compile to predicated instructions, where
   // selects would be: 2.10 -> 2.05 ms on 20,011 positions with 4.0 M playouts)
   uint32_t a = p.lo_a, b = p.lo_b, at = kOffset, sel = kQuarters;
@@ -608,15 +610,13 @@ GA_HD int play_ply_heuristic(RotBoard &b, BlockDraws &rs, bool men_now, bool kin
         big |= (rotl(from, turn_of(v, from, place)) & oppk) ? 1u << c : 0u;
       }
     } else {
-      // the four squares of the row before the last: their moves are the
-      // list's last but for the last row's
+      // the four squares of the row before the last, whose moves are the first of
+      // the last two rows'
       constexpr uint32_t F = 0x00041041u, at = kOffset + 24u;
       const Masks m = masks(b, v);
       const uint32_t q = (rotr(m.m0, at) & F) + (rotr(m.m1, at) & F) + (rotr(m.m2, at) & F) + (rotr(m.m3, at) & F);
       const uint32_t t = rotr(ready, at) & F;
-      constexpr uint32_t last = kFarRow;
-      uint32_t pos = n - (uint32_t)(popc(m.m0 & last) + popc(m.m1 & last) + popc(m.m2 & last) + popc(m.m3 & last)) -
-                     ((q * F >> 18) & 63u);
+      uint32_t pos = n - (uint32_t)(popc(p.hi_a & ~kQuarters) + popc(p.hi_b & ~kQuarters));  // the last two rows'
 GA_UNROLL
       for (uint32_t c = 0; c < 4; c++) {
         const uint32_t cnt = (q >> (6u * c)) & 7u;
@@ -634,6 +634,9 @@ GA_UNROLL
     const uint32_t pair = rs.k >> 1, skip = pair & 1u;  // two draws per move: k is even
     const uint32_t steps = loop_n((skip + n + 1u) >> 1);
     int32_t bw = INT32_MIN;
+#if defined(__CUDACC__)
+#pragma unroll 2  // two blocks in flight: 841 -> 814 us on the benchmark batch (four: 873)
+#endif
     for (uint32_t t = 0; t < steps; t++) {
       uint32_t c[4];
       rs.block((pair >> 1) + t, c);

@@ -102,13 +102,15 @@ struct gpuai_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   int sms = 0;
-  // threads per block by policy: the uniform random kernel runs 512-thread blocks (2 per SM; ~1 % faster
+  // threads per block by policy (launch_shape takes others for small batches): the uniform random kernel runs 512-thread blocks (2 per SM; ~1 % faster
   // than 4 x 256 on 64 x 4,096 batches, equal on large ones: a block packs its games over 16 warps when
   // the work runs out); the 80-register reference-heuristic kernel fits 3 x 256 per SM
   int block[3] = {2 * ga::kPlayoutBlock, ga::kPlayoutBlock, ga::kPlayoutBlock};
   int blocks_per_sm[3] = {0, 0, 0};  // resident blocks per SM used for the grid
   int max_blocks_per_sm[3] = {0, 0, 0};
   int layout[3] = {ga::kLayoutThread, ga::kLayoutThread, ga::kLayoutThread};
+  bool chosen[3] = {false, false, false};  // launch shape or layout set by the caller
+  int small_blocks_per_sm[3][2] = {};      // resident blocks of 128 and 256 threads (0: not asked yet)
   Control *ctl = nullptr;  // device
   Control last_host{};      // control block of the last host-buffer call, as read back
   bool last_was_host = false;
@@ -134,12 +136,30 @@ int set_device(gpuai_ctx *ctx) {
   return GPUAI_OK;
 }
 
-// Blocks of a launch: a block per playout, up to the resident ones (the kernel
-// deals a small batch out over them).
-int grid_for(gpuai_ctx *ctx, int policy, uint32_t total) {
-  const long long resident = (long long)ctx->sms * ctx->blocks_per_sm[policy];
-  const long long g = total < resident ? total : resident;
-  return (int)(g < 1 ? 1 : g);
+// Launch shape of `total` playouts: the caller's, or by size.  A batch that fits
+// the GPU's lanes has no steady state, in which the uniform random policy's wide
+// blocks pay (262,144 playouts: 315 us with 512 threads, 325 with 256), and its
+// blocks' barriers and packing cost less with fewer warps: 140,000 playouts
+// 194 us with 256 threads, 209 with 512; 16,000 150 against 156; with a handful
+// of games per SM 128 threads are better still (1000 playouts of one each 112,
+// 117 with 256 or 512; eps-greedy 149, 153, 160).  The grid is a block per
+// playout up to the resident ones (the kernel deals a small batch out over them).
+int launch_shape(gpuai_ctx *ctx, int policy, uint32_t total, int *block, int *grid) {
+  *block = ctx->block[policy];
+  int per_sm = ctx->blocks_per_sm[policy];
+  if (!ctx->chosen[policy]) {
+    const uint32_t lanes = (uint32_t)ctx->sms * (uint32_t)(ctx->blocks_per_sm[policy] * ctx->block[policy]);
+    const int which = total <= 8u * (uint32_t)ctx->sms ? 0 : (total <= lanes ? 1 : 2);
+    if (which < 2) {
+      *block = which == 0 ? 128 : 256;
+      int &cached = ctx->small_blocks_per_sm[policy][which];
+      if (cached == 0) CK(ga::playout_occupancy(policy, *block, &cached), "occupancy query");
+      per_sm = cached < 1 ? 1 : cached;
+    }
+  }
+  const long long resident = (long long)ctx->sms * per_sm, g = total < resident ? total : resident;
+  *grid = (int)(g < 1 ? 1 : g);
+  return GPUAI_OK;
 }
 
 // Launch on device buffers; ctx->mu held, device current.  ctl is the work
@@ -161,8 +181,10 @@ int launch_device(gpuai_ctx *ctx, const gpuai_board *d_pos, const uint32_t *d_of
   a.counter = &ctl->counter;
   a.status = &ctl->status;
   a.plies = &ctl->plies;
-  CK(ga::launch_playouts(a, policy, ctx->block[policy], grid_for(ctx, policy, total), s, ctx->layout[policy]),
-     "playout kernel launch");
+  int block = 0, grid = 0;
+  const int rc = launch_shape(ctx, policy, total, &block, &grid);
+  if (rc) return rc;
+  CK(ga::launch_playouts(a, policy, block, grid, s, ctx->layout[policy]), "playout kernel launch");
   return GPUAI_OK;
 }
 
@@ -246,6 +268,7 @@ int gpuai_set_launch(gpuai_ctx *ctx, int32_t policy, int32_t block_threads, int3
   CK(ga::playout_occupancy(policy, block_threads, &maxb, ctx->layout[policy]), "occupancy query");
   if (maxb < 1) return fail(GPUAI_ERR_INVALID, "gpuai_set_launch: block of %d threads cannot be resident", block_threads);
   if (blocks_per_sm < 0) return fail(GPUAI_ERR_INVALID, "gpuai_set_launch: negative blocks_per_sm");
+  ctx->chosen[policy] = true;
   ctx->block[policy] = block_threads;
   ctx->max_blocks_per_sm[policy] = maxb;
   ctx->blocks_per_sm[policy] = (blocks_per_sm == 0 || blocks_per_sm > maxb) ? maxb : blocks_per_sm;
@@ -265,6 +288,7 @@ int gpuai_set_layout(gpuai_ctx *ctx, int32_t policy, int32_t layout) {
   int maxb = 0;
   CK(ga::playout_occupancy(policy, ctx->block[policy], &maxb, layout), "occupancy query");
   if (maxb < 1) return fail(GPUAI_ERR_INVALID, "gpuai_set_layout: the kernel cannot be resident");
+  ctx->chosen[policy] = true;
   ctx->layout[policy] = layout;
   ctx->max_blocks_per_sm[policy] = maxb;
   ctx->blocks_per_sm[policy] = maxb;

@@ -138,7 +138,6 @@ struct Epi {
   const float *r1_row = nullptr, *r1_col = nullptr;
   const float *vdot_w = nullptr, *vdot_b = nullptr;
   float *vdot_out = nullptr;
-  float *vdot_tanh = nullptr;  // optional, with kEpiVsum: tanh of vdot_out
   float *vdot_part = nullptr;  // [2][vdot_ld] per-tile partial sums of the value head
   uint32_t vdot_ld = 0;
 };
@@ -438,11 +437,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (bn == 256u) g.e.vdot_part[(size_t)half * g.e.vdot_ld + row] = vs0 + vs1;
     else if (half == 0) g.e.vdot_part[(size_t)blockIdx.y * g.e.vdot_ld + row] = vpart[trow] + vpart[kBM + trow];
   }
-  if ((g.e.flags & kEpiVsum) && blockIdx.y == 0 && half == 0 && row_ok) {  // the two tiles' sums, in order
-    const float v = (g.e.vdot_part[row] + g.e.vdot_part[g.e.vdot_ld + row]) + g.e.vdot_b[0];
-    g.e.vdot_out[row] = v;
-    if (g.e.vdot_tanh) g.e.vdot_tanh[row] = tanhf(v);
-  }
+  if ((g.e.flags & kEpiVsum) && blockIdx.y == 0 && half == 0 && row_ok)  // the two tiles' sums, in order
+    g.e.vdot_out[row] = (g.e.vdot_part[row] + g.e.vdot_part[g.e.vdot_ld + row]) + g.e.vdot_b[0];
   if (*s_err) {
     if (threadIdx.x == 0) {
       atomicOr(g.status, kStatusNetWait);
@@ -883,6 +879,11 @@ __global__ void adam_kernel(AdamArgs a) {
   }
 }
 
+__global__ void tanh_kernel(const float *x, uint32_t n, float *y) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) y[i] = tanhf(x[i]);
+}
+
 // ---- training labels
 
 constexpr uint32_t kLabelSlots = kMaxMoves;  // child slots per position
@@ -1104,11 +1105,8 @@ namespace {
 
 // Forward through the three layers; with `train`, also the transposed
 // activations the backward pass reads.
-// The products launch early (programmatic dependent launch) but for calls whose
-// row count is on the device, which their kernels read first.
 cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards, uint32_t n, const uint32_t *dev_n,
-                         uint32_t rows, uint32_t *status, bool train, cudaStream_t s, float *value = nullptr) {
-  const bool pdl = dev_n == nullptr;
+                         uint32_t rows, uint32_t *status, bool train, cudaStream_t s) {
   const float *P = net->params;
   features_kernel<<<(rows * kChunks + 255) / 256, 256, 0, s>>>(boards, n, dev_n, rows, w.X, train ? net->Xt : nullptr,
                                                      net->rows);
@@ -1121,7 +1119,7 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   e1.ld_b = kH;
   e1.out_t = net->H1t;
   e1.ld_t = net->rows;
-  if ((e = gemm(w.mX, net->mW1, rows, kH, kBnF1, kInPad / kBK, 1, dev_n, status, e1, s, pdl, true)) != cudaSuccess)
+  if ((e = gemm(w.mX, net->mW1, rows, kH, kBnF1, kInPad / kBK, 1, dev_n, status, e1, s, train, true)) != cudaSuccess)
     return e;
   Epi e2 = e1;
   e2.flags |= kEpiVdot;
@@ -1135,7 +1133,7 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   // idle, in 256-column tiles once the row blocks alone fill the SMs
   const bool wide2 = rows / kBM >= sm_count();
   if ((e = gemm(w.mH1, wide2 ? net->mW2w : net->mW2, rows, kH, wide2 ? 2u * kBnF2 : kBnF2, kH / kBK, 1, dev_n, status,
-                e2, s, pdl, true)) != cudaSuccess)
+                e2, s, train, true)) != cudaSuccess)
     return e;
   Epi e3;
   e3.flags = kEpiBias | kEpiVsum | (w.logits_b ? kEpiB16 : kEpiF32);
@@ -1144,12 +1142,11 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   e3.vdot_ld = w.rows;
   e3.vdot_b = P + oBV;
   e3.vdot_out = w.vraw;
-  e3.vdot_tanh = value;
   e3.out_f32 = w.logits;
   e3.ld_f32 = kOut;
   e3.out_b = w.logits_b;
   e3.ld_b = kOut;
-  return gemm(w.mH2, net->mW3, rows, kOut, kBnF3, kH / kBK, 1, dev_n, status, e3, s, pdl, true);
+  return gemm(w.mH2, net->mW3, rows, kOut, kBnF3, kH / kBK, 1, dev_n, status, e3, s, train, true);
 }
 
 // Forward + backward on rows [0, n) of the training workspace; gradients are
@@ -1594,8 +1591,9 @@ int gpuai_net_forward(gpuai_net *net, const gpuai_board *boards, uint32_t n, flo
   for (uint32_t done = 0; done < n;) {
     const uint32_t c = n - done < net->rows ? n - done : net->rows;
     NCK(cudaMemcpyAsync(net->in_boards, boards + done, c * sizeof(gpuai_board), cudaMemcpyHostToDevice, s), "H2D");
-    NCK(forward_impl(net, net->fw, net->in_boards, c, nullptr, round128(c), net->status, false, s, net->value),
-        "forward");
+    NCK(forward(net, net->fw, net->in_boards, c, nullptr, net->status, s), "forward");
+    tanh_kernel<<<(c + 255) / 256, 256, 0, s>>>(net->fw.vraw, c, net->value);
+    NCK(cudaGetLastError(), "tanh");
     NCK(cudaMemcpyAsync(value + done, net->value, c * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     if (logits)
       NCK(cudaMemcpyAsync(logits + (size_t)done * kOut, net->fw.logits, (size_t)c * kOut * sizeof(float),

@@ -34,8 +34,9 @@
 // Every reduction has a fixed order, so a training run is reproducible.
 // The chain features .. F3, loss, B1, B3, B5, Adam runs on the network's stream,
 // each kernel launched while the one before it drains (programmatic
-// dependent launch) and set up before it waits for it; B2 and its row sums run on a second stream, B4 and the
-// remaining row sums on a third.  dZ3 and dZ3^T are all zero between steps:
+// dependent launch) and set up before it waits for it; B2 and its row sums run
+// on a second stream, B4 and the remaining row sums on a third.  dZ3 and dZ3^T
+// are all zero between steps:
 // the loss writes at most 32 entries of a row and clear_dz3_kernel zeroes
 // them again once B1 and B2 have read them.
 #include "net.h"
@@ -138,6 +139,7 @@ struct Epi {
   const float *r1_row = nullptr, *r1_col = nullptr;
   const float *vdot_w = nullptr, *vdot_b = nullptr;
   float *vdot_out = nullptr;
+  float *vdot_tanh = nullptr;  // optional, with kEpiVsum: tanh of vdot_out
   float *vdot_part = nullptr;  // [2][vdot_ld] per-tile partial sums of the value head
   uint32_t vdot_ld = 0;
 };
@@ -437,8 +439,11 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (bn == 256u) g.e.vdot_part[(size_t)half * g.e.vdot_ld + row] = vs0 + vs1;
     else if (half == 0) g.e.vdot_part[(size_t)blockIdx.y * g.e.vdot_ld + row] = vpart[trow] + vpart[kBM + trow];
   }
-  if ((g.e.flags & kEpiVsum) && blockIdx.y == 0 && half == 0 && row_ok)  // the two tiles' sums, in order
-    g.e.vdot_out[row] = (g.e.vdot_part[row] + g.e.vdot_part[g.e.vdot_ld + row]) + g.e.vdot_b[0];
+  if ((g.e.flags & kEpiVsum) && blockIdx.y == 0 && half == 0 && row_ok) {  // the two tiles' sums, in order
+    const float v = (g.e.vdot_part[row] + g.e.vdot_part[g.e.vdot_ld + row]) + g.e.vdot_b[0];
+    g.e.vdot_out[row] = v;
+    if (g.e.vdot_tanh) g.e.vdot_tanh[row] = tanhf(v);
+  }
   if (*s_err) {
     if (threadIdx.x == 0) {
       atomicOr(g.status, kStatusNetWait);
@@ -879,11 +884,6 @@ __global__ void adam_kernel(AdamArgs a) {
   }
 }
 
-__global__ void tanh_kernel(const float *x, uint32_t n, float *y) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] = tanhf(x[i]);
-}
-
 // ---- training labels
 
 constexpr uint32_t kLabelSlots = kMaxMoves;  // child slots per position
@@ -1105,8 +1105,14 @@ namespace {
 
 // Forward through the three layers; with `train`, also the transposed
 // activations the backward pass reads.
+// The products launch early (programmatic dependent launch) but for calls whose
+// row count is on the device, which their kernels read first.  These chains are
+// launch latency up to a few thousand boards: with the tanh in the last epilogue
+// instead of a kernel of its own, a call takes 59 instead of 71 us for 1 board,
+// 148 instead of 161 for 1000, 425 instead of 436 for 4000.
 cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards, uint32_t n, const uint32_t *dev_n,
-                         uint32_t rows, uint32_t *status, bool train, cudaStream_t s) {
+                         uint32_t rows, uint32_t *status, bool train, cudaStream_t s, float *value = nullptr) {
+  const bool pdl = dev_n == nullptr;
   const float *P = net->params;
   features_kernel<<<(rows * kChunks + 255) / 256, 256, 0, s>>>(boards, n, dev_n, rows, w.X, train ? net->Xt : nullptr,
                                                      net->rows);
@@ -1119,7 +1125,7 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   e1.ld_b = kH;
   e1.out_t = net->H1t;
   e1.ld_t = net->rows;
-  if ((e = gemm(w.mX, net->mW1, rows, kH, kBnF1, kInPad / kBK, 1, dev_n, status, e1, s, train, true)) != cudaSuccess)
+  if ((e = gemm(w.mX, net->mW1, rows, kH, kBnF1, kInPad / kBK, 1, dev_n, status, e1, s, pdl, true)) != cudaSuccess)
     return e;
   Epi e2 = e1;
   e2.flags |= kEpiVdot;
@@ -1133,7 +1139,7 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   // idle, in 256-column tiles once the row blocks alone fill the SMs
   const bool wide2 = rows / kBM >= sm_count();
   if ((e = gemm(w.mH1, wide2 ? net->mW2w : net->mW2, rows, kH, wide2 ? 2u * kBnF2 : kBnF2, kH / kBK, 1, dev_n, status,
-                e2, s, train, true)) != cudaSuccess)
+                e2, s, pdl, true)) != cudaSuccess)
     return e;
   Epi e3;
   e3.flags = kEpiBias | kEpiVsum | (w.logits_b ? kEpiB16 : kEpiF32);
@@ -1142,11 +1148,12 @@ cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards
   e3.vdot_ld = w.rows;
   e3.vdot_b = P + oBV;
   e3.vdot_out = w.vraw;
+  e3.vdot_tanh = value;
   e3.out_f32 = w.logits;
   e3.ld_f32 = kOut;
   e3.out_b = w.logits_b;
   e3.ld_b = kOut;
-  return gemm(w.mH2, net->mW3, rows, kOut, kBnF3, kH / kBK, 1, dev_n, status, e3, s, train, true);
+  return gemm(w.mH2, net->mW3, rows, kOut, kBnF3, kH / kBK, 1, dev_n, status, e3, s, pdl, true);
 }
 
 // Forward + backward on rows [0, n) of the training workspace; gradients are
@@ -1591,9 +1598,8 @@ int gpuai_net_forward(gpuai_net *net, const gpuai_board *boards, uint32_t n, flo
   for (uint32_t done = 0; done < n;) {
     const uint32_t c = n - done < net->rows ? n - done : net->rows;
     NCK(cudaMemcpyAsync(net->in_boards, boards + done, c * sizeof(gpuai_board), cudaMemcpyHostToDevice, s), "H2D");
-    NCK(forward(net, net->fw, net->in_boards, c, nullptr, net->status, s), "forward");
-    tanh_kernel<<<(c + 255) / 256, 256, 0, s>>>(net->fw.vraw, c, net->value);
-    NCK(cudaGetLastError(), "tanh");
+    NCK(forward_impl(net, net->fw, net->in_boards, c, nullptr, round128(c), net->status, false, s, net->value),
+        "forward");
     NCK(cudaMemcpyAsync(value + done, net->value, c * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     if (logits)
       NCK(cudaMemcpyAsync(logits + (size_t)done * kOut, net->fw.logits, (size_t)c * kOut * sizeof(float),

@@ -60,6 +60,7 @@ namespace ga {
 namespace {
 
 constexpr uint32_t kExpanded = 1u, kTerminal = 2u, kEvaluated = 4u;  // node state bits (info.y >> 16)
+constexpr uint32_t kFull = 0xffffffffu;  // all lanes of a warp
 constexpr int kMaxSelectDepth = 512;
 constexpr uint32_t kStatusSelectDepth = 8u;
 // Frontier entries whose expansions take nodes together in a step with Q leaves
@@ -70,6 +71,7 @@ constexpr float kUcbC = 1.41421356f;
 constexpr int kMaxChildren = 64;  // moves per position handled by split_slots
 constexpr uint32_t kUnits = 64;   // learned searches: visit units per leaf slot (score2 = units * (1 + value))
 constexpr uint32_t kPriors = 32;  // stored priors per node (more moves: uniform priors)
+constexpr uint32_t kAhead = 4;    // slots whose exploration terms split_puct prepares together (2 and 8: slower)
 constexpr float kFpuReduction = 0.1f;  // unvisited child's Q = parent's Q - this
 constexpr float kTerminalLeaf = 2.0f;  // leaf value marking a finished game
 
@@ -215,32 +217,42 @@ __device__ __forceinline__ void expand_group(const Pool &p, const Board &b, int3
 // src/mcts.cpp:95-136): untried children share them equally; otherwise in
 // proportion to UCB1 weights rounded down; the remainder goes one each to the
 // heaviest children (first on ties).  Weights that sum to zero count as
-// equal.  Fills give[0..k) and returns the number of children given slots.
+// equal.
 // The weights use the correctly rounded operations of detmath.cuh in a fixed
 // order, so the CPU restatement (oracle/search.py) reproduces every split.
-__device__ __forceinline__ float ucb_weight(uint4 ci, float lnN) {
-  const float mean = dm::div(dm::mul(0.5f, (float)ci.w), (float)ci.z);
-  return dm::add(mean, dm::mul(kUcbC, dm::sqrt_(dm::div(lnN, (float)ci.z))));
+// A quotient with a zero numerator takes the division's slow path, and its
+// whole warp with it (330 against 58 cycles): where there is nothing to divide,
+// here and in split_puct, lanes divide 1 and drop the result.
+__device__ __forceinline__ float ucb_weight(uint32_t visits, uint32_t score2, float lnN) {
+  const float n = (float)(visits ? visits : 1u);
+  const float mean = dm::div(score2 ? dm::mul(0.5f, (float)score2) : 1.0f, n);
+  return dm::add(score2 ? mean : 0.0f, dm::mul(kUcbC, dm::sqrt_(dm::div(lnN, n))));
 }
 
 // The children of a node on a group of G lanes, child c on lane c % G as its
 // (c / G)-th of J: what a split reads of them, and the slots it
 // gives.  The k children of a node just expanded (fresh) are not read: none has
-// been visited.
+// been visited.  `own` takes a lane's first child from v0 and h0.
 template <int J, uint32_t G>
 struct Children {
   static constexpr int kPerLane = J;
+  static constexpr uint32_t kLanes = G;
   uint32_t link[J], state[J], visits[J], score2[J], give[J];
   float prior[J];
   __device__ __forceinline__ void load(const Pool &p, int32_t first, int k, bool fresh, uint32_t gl,
-                                       const __half *priors) {
+                                       const __half *priors, bool own, const uint4 &v0, __half h0) {
 #pragma unroll
     for (int j = 0; j < J; j++) {
       const int c = (int)gl + (int)G * j;
       uint4 v = make_uint4(0xffffffffu, 0u, 0u, 0u);
       __half h = __float2half(0.0f);
-      if (c < k && !fresh) v = p.info[first + c];
-      if (c < k && priors) h = priors[c];
+      if (j == 0 && own) {
+        v = v0;
+        h = h0;
+      } else {
+        if (c < k && !fresh) v = p.info[first + c];
+        if (c < k && priors) h = priors[c];
+      }
       link[j] = v.x;
       state[j] = v.y;
       visits[j] = v.z;
@@ -255,7 +267,7 @@ struct Children {
     const uint32_t lower = group & ((1u << (threadIdx.x & 31u)) - 1u);
 #pragma unroll
     for (int j = 0; j < J; j++) {
-      const uint32_t got = __ballot_sync(group, give[j] != 0) & group;
+      const uint32_t got = __ballot_sync(kFull, give[j] != 0) & group;
       if (give[j]) {
         const uint32_t w = at + __popc(got & lower);
         t_node[w] = first + (int32_t)(gl + G * j);
@@ -268,7 +280,10 @@ struct Children {
 };
 
 // Splits T slots over the k children of a node; `lane0` is the group's first
-// lane of the warp.
+// lane of the warp.  Every lane of the warp calls it, a group without a node
+// with k = T = 0: an operation of the warp with a mask per group runs once for
+// each mask (four groups of eight lanes: a shuffle 131 against 50 cycles, a
+// vote 395 against 56, a reduction 516 against 56).
 template <int J, uint32_t G>
 __device__ __forceinline__ void split_slots(Children<J, G> &ch, int k, uint32_t parent_visits, uint32_t T, uint32_t gl,
                                             uint32_t lane0, uint32_t group) {
@@ -278,51 +293,47 @@ __device__ __forceinline__ void split_slots(Children<J, G> &ch, int k, uint32_t 
 #pragma unroll
   for (int j = 0; j < J; j++) {
     const bool child = (int)(gl + G * j) < k, fresh = child && ch.visits[j] == 0;
-    w[j] = fresh ? 3.0e38f : -2.0f;  // no child: below every weight
-    if (child && !fresh) w[j] = ucb_weight(make_uint4(0u, 0u, ch.visits[j], ch.score2[j]), lnN);
-    untried += __popc(__ballot_sync(group, fresh) & group);
+    w[j] = ucb_weight(ch.visits[j], ch.score2[j], lnN);
+    if (!child || fresh) w[j] = child ? 3.0e38f : -2.0f;  // no child: below every weight
+    untried += __popc(__ballot_sync(kFull, fresh) & group);
   }
-  if (untried == 0) {  // the sum in child order
+  // the sum in child order, and how many children are heavier (first on ties)
+  uint32_t heavier[J];
 #pragma unroll
-    for (int j = 0; j < J; j++)
+  for (int j = 0; j < J; j++) heavier[j] = 0;
 #pragma unroll
-      for (uint32_t c = 0; c < G; c++) {
-        const float x = __shfl_sync(group, w[j], lane0 + c);
-        if ((int)(c + G * j) < k) wsum = dm::add(wsum, x);
-      }
+  for (int i = 0; i < J; i++) {
+    const int here = k - (int)G * i;  // k is the warp's where G is 32
+#pragma unroll (G < 32u ? (int)G : 4)
+    for (int c = 0; c < (G < 32u ? (int)G : here); c++) {
+      const float x = __shfl_sync(kFull, w[i], lane0 + c);
+      wsum = dm::add(wsum, c < here ? x : 0.0f);
+#pragma unroll
+      for (int j = 0; j < J; j++)
+        heavier[j] += (uint32_t)((x > w[j]) | ((x == w[j]) & (c + (int)G * i < (int)(gl + G * j))));
+    }
   }
   const bool equal = untried == 0 && !(wsum > 0.0f);
-  const float whole = equal ? (float)k : wsum;
+  const float whole = untried || k == 0 ? 1.0f : (equal ? (float)k : wsum);
   const uint32_t each = untried ? T / untried : 0u;
   uint32_t assigned = 0;
 #pragma unroll
   for (int j = 0; j < J; j++) {
     const bool child = (int)(gl + G * j) < k;
-    if (equal && child) w[j] = 1.0f;
-    if (child) {
-      if (untried) ch.give[j] = ch.visits[j] == 0 ? each : 0u;
-      else ch.give[j] = (uint32_t)dm::mul((float)T, dm::div(w[j], whole));
+    if (equal && child) {
+      w[j] = 1.0f;
+      heavier[j] = gl + G * j;
     }
+    const uint32_t share = (uint32_t)dm::mul((float)T, dm::div(child && !untried ? w[j] : 1.0f, whole));
+    if (child) ch.give[j] = untried ? (ch.visits[j] == 0 ? each : 0u) : share;
     assigned += ch.give[j];
   }
-  assigned = __reduce_add_sync(group, assigned);
-  if (assigned < T) {  // the remainder (fewer than k), one each to the heaviest, first on ties
-    uint32_t heavier[J];
 #pragma unroll
-    for (int j = 0; j < J; j++) heavier[j] = 0;
+  for (uint32_t o = 1; o < G; o <<= 1) assigned += __shfl_xor_sync(kFull, assigned, o);
+  const uint32_t rest = assigned < T ? T - assigned : 0u;  // fewer than k: one each to the heaviest
 #pragma unroll
-    for (int i = 0; i < J; i++)
-#pragma unroll
-      for (uint32_t c = 0; c < G; c++) {
-        const float x = __shfl_sync(group, w[i], lane0 + c);
-#pragma unroll
-        for (int j = 0; j < J; j++)
-          heavier[j] += x > w[j] || (x == w[j] && c + G * i < gl + G * j) ? 1u : 0u;
-      }
-#pragma unroll
-    for (int j = 0; j < J; j++)
-      if ((int)(gl + G * j) < k && heavier[j] < T - assigned) ch.give[j]++;
-  }
+  for (int j = 0; j < J; j++)
+    if ((int)(gl + G * j) < k && heavier[j] < rest) ch.give[j]++;
 }
 
 // Learned searches: splits T slots over the k children of node n one slot at
@@ -333,59 +344,100 @@ __device__ __forceinline__ void split_slots(Children<J, G> &ch, int k, uint32_t 
 // has not been evaluated), N = n's visits and n the child's, in leaf slots.
 // A warp takes a node, a child per lane (two for more than 32).  A slot is a
 // chain of a few operations: the square roots of 32 slots are taken at once, a
-// lane each, a child's next exploration term is ready before the child is
-// chosen, and the scores (never negative) are compared as whole numbers by one
-// reduction.
+// lane each, the exploration terms that the next kAhead slots can need together,
+// a child's next score, chosen or not, is ready before one is chosen, and the
+// scores (never negative) are compared as whole numbers by one reduction.  300
+// cycles a slot with a division after each choice, 200 now.
 template <int J>
 __device__ __forceinline__ void split_puct(Children<J, 32> &ch, int k, bool priors, uint32_t parent_visits,
                                            uint32_t parent_score2, uint32_t T, float c_puct, uint32_t lane) {
-  constexpr uint32_t kFull = 0xffffffffu;
   if (k == 1) {
     if (lane == 0) ch.give[0] = T;
     return;
   }
-  float q[J], u[J], un[J], pr[J], nv[J];
-  const float fpu =
-      parent_visits
-          ? fmaxf(0.0f, dm::sub(dm::sub(1.0f, dm::div(dm::mul(0.5f, (float)parent_score2), (float)parent_visits)),
-                                kFpuReduction))
-          : 0.5f;
-  const float uniform = dm::div(1.0f, (float)k);
+  const float half1 = dm::mul(0.5f, (float)parent_score2), all1 = (float)(parent_visits ? parent_visits : 1u);
+  float q[J], pr[J], nv[J];
+#pragma unroll
+  for (int j = 0; j < J; j++) {  // the parent's mean on lane 31, where it has no child, else apart
+    const bool parent = J == 1 && (int)lane >= k, tried = ch.visits[j] != 0;
+    q[j] = dm::div(parent ? half1 : (tried ? dm::mul(0.5f, (float)ch.score2[j]) : 1.0f),
+                   parent ? all1 : (tried ? (float)ch.visits[j] : 1.0f));
+  }
+  const float mean = J == 1 && k < 32 ? __shfl_sync(kFull, q[0], 31) : dm::div(half1, all1);
+  const float fpu = parent_visits ? fmaxf(0.0f, dm::sub(dm::sub(1.0f, mean), kFpuReduction)) : 0.5f;
+  const float uniform = priors ? 0.0f : dm::div(1.0f, (float)k);
 #pragma unroll
   for (int j = 0; j < J; j++) {
-    const int c = (int)lane + 32 * j;
-    q[j] = ch.visits[j] ? dm::div(dm::mul(0.5f, (float)ch.score2[j]), (float)ch.visits[j]) : fpu;
+    if (ch.visits[j] == 0) q[j] = fpu;
+    if ((int)lane + 32 * j >= k) q[j] = -4.0e18f;  // no child: below every score
     nv[j] = dm::add(1.0f, (float)(ch.visits[j] / kUnits));
-    pr[j] = c < k ? dm::mul(c_puct, priors ? ch.prior[j] : uniform) : 0.0f;
-    u[j] = dm::div(pr[j], nv[j]);  // exploration term without the sqrt(N) factor
-    nv[j] = dm::add(nv[j], 1.0f);
-    un[j] = dm::div(pr[j], nv[j]);  // ... after one more slot
+    pr[j] = (int)lane + 32 * j < k ? dm::mul(c_puct, priors ? ch.prior[j] : uniform) : 1.0f;
   }
   const float N = (float)(parent_visits / kUnits);
   float roots = 0.0f;
-  for (uint32_t t = 0; t < T; t++) {
-    if (t % 32u == 0) roots = dm::sqrt_(dm::add(dm::add(N, (float)(t + lane)), 1.0f));
-    const float sq = __shfl_sync(kFull, roots, t % 32u);
-    uint32_t top = 0, best = 0;  // score + 1 (0: no child), child
+  const uint32_t lower = (1u << lane) - 1u;
+  for (uint32_t t = 0; t < T;) {
+    // the children's exploration terms, without the sqrt(N) factor, for as many slots as the next kAhead can give one
+    const uint32_t ahead = min(T - t, kAhead);
+    float u[J][kAhead + 1], sq[kAhead];
+    if (J == 1 && k <= 16 && ahead > 1) {
+      // few children: the lanes beyond them take later terms of the same quotient
+      const uint32_t width = k <= 8 ? 8u : 16u, c = lane & (width - 1u), later = lane / width;
+      const float p0 = __shfl_sync(kFull, pr[0], c);
+      const float n0 = __shfl_sync(kFull, nv[0], c), n1 = dm::add(n0, 1.0f), n2 = dm::add(n1, 1.0f),
+                  n3 = dm::add(n2, 1.0f);
+      if (k <= 8) {
+        const float d = dm::div(p0, later & 2u ? (later & 1u ? n3 : n2) : (later & 1u ? n1 : n0));
 #pragma unroll
-    for (int j = 0; j < J; j++) {
-      const uint32_t key =
-          (int)lane + 32 * j < k ? __float_as_uint(dm::add(dm::mul(sq, u[j]), q[j])) + 1u : 0u;
-      const uint32_t m = __reduce_max_sync(kFull, key);
-      const uint32_t first = __ffs(__ballot_sync(kFull, key == m)) - 1u + 32u * j;
-      if (m > top) {
-        top = m;
-        best = first;
+        for (uint32_t i = 0; i < kAhead; i++) u[0][i] = __shfl_sync(kFull, d, c + 8u * i);
+      } else {
+        const float a = dm::div(p0, later ? n1 : n0), b = dm::div(p0, later ? n3 : n2);
+#pragma unroll
+        for (uint32_t i = 0; i < kAhead; i++) u[0][i] = __shfl_sync(kFull, i < 2 ? a : b, c + 16u * (i & 1u));
+      }
+      u[0][kAhead] = 0.0f;
+    } else {
+#pragma unroll
+      for (int j = 0; j < J; j++) {
+        float n = nv[j];
+#pragma unroll
+        for (uint32_t i = 0; i < kAhead; i++) {
+          u[j][i] = i < ahead ? dm::div(pr[j], n) : 0.0f;
+          n = dm::add(n, 1.0f);
+        }
+        u[j][kAhead] = 0.0f;
       }
     }
+    if (t % 32u == 0) roots = dm::sqrt_(dm::add(dm::add(N, (float)(t + lane)), 1.0f));
 #pragma unroll
-    for (int j = 0; j < J; j++)
-      if (best == lane + 32u * j) {
-        ch.give[j]++;
-        u[j] = un[j];
-        nv[j] = dm::add(nv[j], 1.0f);
-        un[j] = dm::div(pr[j], nv[j]);
+    for (uint32_t i = 0; i < kAhead; i++) sq[i] = __shfl_sync(kFull, roots, (t + i) % 32u);
+    int key[J];
+#pragma unroll
+    for (int j = 0; j < J; j++) key[j] = __float_as_int(dm::add(dm::mul(sq[0], u[j][0]), q[j]));
+#pragma unroll
+    for (uint32_t i = 0; i < kAhead; i++) {
+      if (i >= ahead) break;
+      int top = key[0];
+#pragma unroll
+      for (int j = 1; j < J; j++) top = max(top, key[j]);
+      top = __reduce_max_sync(kFull, top);
+      uint32_t before = 0;  // children of lower index with the same score
+#pragma unroll
+      for (int j = 0; j < J; j++) {
+        const float next = i + 1 < kAhead ? sq[i + 1 < kAhead ? i + 1 : i] : 0.0f;
+        const int passed = __float_as_int(dm::add(dm::mul(next, u[j][0]), q[j])),
+                  taken = __float_as_int(dm::add(dm::mul(next, u[j][1]), q[j]));
+        const uint32_t same = __ballot_sync(kFull, key[j] == top);
+        const bool mine = (key[j] == top) & ((before | (same & lower)) == 0);
+        before |= same;
+        ch.give[j] += mine ? 1u : 0u;
+        nv[j] = mine ? dm::add(nv[j], 1.0f) : nv[j];
+        key[j] = mine ? taken : passed;
+#pragma unroll
+        for (uint32_t a = 0; a < kAhead; a++) u[j][a] = mine ? u[j][a + 1] : u[j][a];
       }
+    }
+    t += ahead;
   }
 }
 
@@ -398,11 +450,13 @@ __device__ __forceinline__ void split_puct(Children<J, 32> &ch, int k, bool prio
 // compaction over the slots makes the next frontier.
 //
 // What bounds it is the latency of a level, so each level's serial stretches
-// are shared out: a group of lanes (eight, a warp for learned searches) expands
-// or splits a node, a child per lane.  A thread per entry that enumerated,
-// loaded and split one child after the other took, with the rest of the step,
-// 13.5 against 11.5 ms for 32 steps of 64 searches x 512 leaves, and 17.5
-// against 11.3 ms for 48 steps of 200 learned searches x 64 leaves.
+// are shared out: a group of lanes (eight, a warp for learned searches and for
+// nodes of more than 16 children) expands or splits a node, a child per lane,
+// whose record is loaded while the node before is split.  A thread per entry
+// that enumerated, loaded and split one child after the other took 152 us for a
+// step of 64 searches x 512 leaves, and 205 us for one of 200 learned searches
+// x 64 leaves; groups that used masks of their own and divided zeros 97 and
+// 70 us; as it stands 56 and 55 us.
 //
 // Node ranges run out by rounds of `round` entries (a warp's below 128 leaves
 // per search, else 128, 256 or 512): an expansion that does not fit what its
@@ -413,7 +467,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
     select_kernel(Pool p, Table t, Leaves l, uint32_t slots, uint32_t ppl, uint32_t round, Learned lrn,
                   uint32_t *status) {
   constexpr int kWarps = T / 32;
-  constexpr uint32_t G = LEARNED ? 32u : 8u;  // lanes that take a node
+  constexpr uint32_t G = LEARNED ? 32u : 8u, kGroups = 32u / G;  // lanes that take a node, nodes a warp takes
   constexpr uint32_t kLeafSlot = 0x80000000u;
   __shared__ int32_t f_node[T];   // the frontier: node, slots, the node's record
   __shared__ uint32_t f_cnt[T];
@@ -423,7 +477,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
   __shared__ uint4 t_info[T];
   __shared__ int32_t s_leaf[T];   // the leaf slots' nodes
   __shared__ uint4 s_board[T];    // boards of the nodes to expand
-  __shared__ uint32_t s_scan[2][kWarps];
+  __shared__ __align__(16) uint32_t s_scan[2][kWarps];
   // the entries that expand or split, for their groups: first child, children | state << 8 | fresh << 31 (0:
   // none), first slot
   __shared__ int32_t s_first[T];
@@ -435,46 +489,47 @@ __global__ void __launch_bounds__(T, 1024 / T)
   if (root < 0) return;  // uniform over the block
   const uint32_t off = t.quota_off[s], q = t.quota_off[s + 1] - off;
   if (q == 0 || !GA_IN_BOUNDS(q <= (uint32_t)T, status)) return;
-  // inclusive prefix sums of a and b over the block's threads, and their totals
-  auto scan2 = [&](uint32_t &a, uint32_t &b, uint32_t &ta, uint32_t &tb) {
-#pragma unroll
-    for (uint32_t o = 1; o < 32; o <<= 1) {
-      const uint32_t x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
-      if (lane >= o) {
-        a += x;
-        b += y;
-      }
-    }
-    if (lane == 31) {
-      s_scan[0][warp] = a;
-      s_scan[1][warp] = b;
-    }
+  // Entries and slots are at most q, a thread each: the warps beyond them take
+  // no part in the scans.  Two sums go in one word (slots, at most 512, below
+  // children, at most 512 * kMaxChildren), and the warps' totals alternate
+  // between two buffers, so that a scan is one barrier.
+  const uint32_t qw = (q + 31u) / 32u;
+  uint32_t buf = 0;
+  if (tid < 2 * kWarps) s_scan[tid / kWarps][tid % kWarps] = 0;
+  // v: the inclusive sums within the warp; returns those over the block
+  auto over_warps = [&](uint32_t v, uint32_t &total) -> uint32_t {
+    if (lane == 31 && warp < qw) s_scan[buf][warp] = v;
     __syncthreads();
-    uint32_t pa = 0, pb = 0;
-    ta = 0;
-    tb = 0;
+    uint32_t before = 0, sum = 0;
 #pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-      const uint32_t va = s_scan[0][w], vb = s_scan[1][w];
-      if ((uint32_t)w < warp) {
-        pa += va;
-        pb += vb;
-      }
-      ta += va;
-      tb += vb;
+    for (int w = 0; w < kWarps; w += 4) {
+      if ((uint32_t)w >= qw) break;
+      const uint4 x = *reinterpret_cast<const uint4 *>(&s_scan[buf][w]);
+      before += ((uint32_t)w < warp ? x.x : 0u) + (w + 1u < warp ? x.y : 0u) + (w + 2u < warp ? x.z : 0u) +
+                (w + 3u < warp ? x.w : 0u);
+      sum += (x.x + x.y) + (x.z + x.w);
     }
-    a += pa;
-    b += pb;
-    __syncthreads();  // s_scan is reused by the next scan
+    buf ^= 1u;
+    total = sum;
+    return v + before;
+  };
+  auto scan = [&](uint32_t v, uint32_t &total) -> uint32_t {
+    if (warp < qw) {
+#pragma unroll
+      for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += x;
+      }
+    }
+    return over_warps(v, total);
   };
   auto block_max = [&](uint32_t x) -> uint32_t {
     x = __reduce_max_sync(0xffffffffu, x);
-    if (lane == 0) s_scan[0][warp] = x;
+    if (lane == 31 && warp < qw) s_scan[buf][warp] = x;
     __syncthreads();
     uint32_t m = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) m = max(m, s_scan[0][w]);
-    __syncthreads();
+    for (uint32_t w = 0; w < qw; w++) m = max(m, s_scan[buf][w]);
+    buf ^= 1u;
     return m;
   };
   uint32_t nf = 1, emitted = 0;
@@ -519,9 +574,10 @@ __global__ void __launch_bounds__(T, 1024 / T)
         leaf = grow == 0;
       }
     }
-    uint32_t sx = slots_here, gx = (uint32_t)grow, stot = 0, gtot = 0;
-    scan2(sx, gx, stot, gtot);
-    const uint32_t at = sx - slots_here;  // the entry's first slot of the level's
+    uint32_t tot;
+    const uint32_t sums = scan(slots_here | ((uint32_t)grow << 16), tot);
+    const uint32_t gx = sums >> 16, stot = tot & 0xffffu, gtot = tot >> 16;
+    const uint32_t at = (sums & 0xffffu) - slots_here;  // the entry's first slot of the level's
     bool fresh = false;
     if (gtot != 0) {  // uniform over the block
       if (node_next + (int64_t)gtot <= node_end) {
@@ -561,27 +617,52 @@ __global__ void __launch_bounds__(T, 1024 / T)
     s_k[tid] = tid < nf && !leaf ? (uint32_t)k | (st << 8) | (fresh ? 0x80000000u : 0u) : 0u;
     s_at[tid] = at;
     __syncthreads();
-    for (uint32_t e = gi; e < nf; e += T / G) {  // uniform over the group
-      const uint32_t ke = s_k[e];
-      if (ke == 0) continue;
-      const int32_t ne = f_node[e], fe = s_first[e];
+    // a lane's child of an entry, loaded while the entry before it is split
+    uint4 next_v = make_uint4(0u, 0u, 0u, 0u);
+    __half next_h = __float2half(0.0f);
+    auto fetch = [&](uint32_t e) {
+      const uint32_t ke = e < nf ? s_k[e] : 0u;
+      next_v = make_uint4(0xffffffffu, 0u, 0u, 0u);
+      if (gl < (ke & 0xffu)) {
+        if (!(ke & 0x80000000u)) next_v = p.info[s_first[e] + (int32_t)gl];
+        if (LEARNED && ((ke >> 8) & kEvaluated)) next_h = p.prior[(size_t)f_node[e] * kPriors + gl];
+      }
+    };
+    fetch(gi);
+    for (uint32_t e0 = warp * kGroups; e0 < nf; e0 += T / G) {  // uniform over the warp
+      const uint32_t e = e0 + gi % kGroups, ke = e < nf ? s_k[e] : 0u;
+      const uint4 v0 = next_v;
+      const __half h0 = next_h;
+      fetch(e + T / G);
       const int kk = (int)(ke & 0xffu);
       const bool fr = (ke & 0x80000000u) != 0;
-      const bool pri = LEARNED && ((ke >> 8) & kEvaluated) && kk <= (int)kPriors;
-      const uint32_t vis = f_info[e].z;
-      auto split = [&](auto &&ch) {
-        constexpr int J = std::remove_reference_t<decltype(ch)>::kPerLane;
-        ch.load(p, fe, kk, fr, gl, pri ? p.prior + (size_t)ne * kPriors : nullptr);
-        if constexpr (LEARNED) split_puct<J>(ch, kk, pri, vis, f_info[e].w, f_cnt[e], lrn.c_puct, lane);
-        else split_slots<J, G>(ch, kk, vis, f_cnt[e], gl, lane0, group);
-        ch.put(fe, t_node, t_cnt, t_info, s_at[e], gl, group);
+      // the groups' nodes (no children and no slots where a group has none here)
+      auto split = [&](auto &&ch, uint32_t at, int k, uint32_t ke, uint32_t gl, uint32_t lane0, uint32_t group) {
+        using C = std::remove_reference_t<decltype(ch)>;
+        const int32_t first = s_first[at];
+        const uint32_t cnt = k ? f_cnt[at] : 0u;
+        const __half *pri = nullptr;
+        if (LEARNED && ((ke >> 8) & kEvaluated) && k <= (int)kPriors) pri = p.prior + (size_t)f_node[at] * kPriors;
+        ch.load(p, first, k, (ke & 0x80000000u) != 0, gl, pri, C::kLanes == G, v0, h0);
+        if constexpr (LEARNED)
+          split_puct<C::kPerLane>(ch, k, pri != nullptr, f_info[at].z, f_info[at].w, cnt, lrn.c_puct, lane);
+        else split_slots(ch, k, f_info[at].z, cnt, gl, lane0, group);
+        ch.put(first, t_node, t_cnt, t_info, s_at[at], gl, group);
       };
-      if (kk <= (int)G) split(Children<1, G>{});
-      else if (kk <= 2 * (int)G) split(Children<2, G>{});
-      else if constexpr (!LEARNED) split(Children<kMaxChildren / (int)G, G>{});
+      const bool many = kk > 2 * (int)G;
+      const int ks = many ? 0 : kk;
+      const uint32_t at_e = ks ? e : 0u;
+      if (__any_sync(kFull, ks > (int)G)) split(Children<2, G>{}, at_e, ks, ke, gl, lane0, group);
+      else if (__any_sync(kFull, ks != 0)) split(Children<1, G>{}, at_e, ks, ke, gl, lane0, group);
+      if constexpr (!LEARNED) {  // nodes of more than 16 children take the warp
+        for (uint32_t left = __ballot_sync(kFull, many && gl == 0); left; left &= left - 1u) {
+          const uint32_t b = e0 + (__ffs(left) - 1u) / G, kb = s_k[b];
+          split(Children<2, 32u>{}, b, (int)(kb & 0xffu), kb, lane, 0u, kFull);
+        }
+      }
       if (fr) {
         const uint4 bv = s_board[e];
-        expand_group<G>(p, Board{bv.x, bv.y, bv.z, bv.w}, ne, fe, kk, gl);
+        expand_group<G>(p, Board{bv.x, bv.y, bv.z, bv.w}, f_node[e], s_first[e], kk, gl);
       }
     }
     __syncthreads();
@@ -589,8 +670,11 @@ __global__ void __launch_bounds__(T, 1024 / T)
     const uint32_t have = tid < stot ? t_cnt[tid] : 0u;
     const int32_t node = tid < stot ? t_node[tid] : 0;
     const bool is_leaf = have == kLeafSlot;
-    uint32_t kx = have != 0 && !is_leaf ? 1u : 0u, lx = is_leaf ? 1u : 0u, ktot = 0, ltot = 0;
-    scan2(kx, lx, ktot, ltot);
+    const uint32_t upto = 0xffffffffu >> (31u - lane);
+    const uint32_t kept = __popc(__ballot_sync(0xffffffffu, have != 0 && !is_leaf) & upto),
+                   left = __popc(__ballot_sync(0xffffffffu, is_leaf) & upto);
+    const uint32_t places = over_warps(kept | (left << 16), tot);
+    const uint32_t kx = places & 0xffffu, lx = places >> 16;
     t_cnt[tid] = 0;
     if (is_leaf) {
       if (GA_IN_BOUNDS(emitted + lx <= q && (uint32_t)node < p.nodes, status)) s_leaf[emitted + lx - 1u] = node;
@@ -599,8 +683,8 @@ __global__ void __launch_bounds__(T, 1024 / T)
       f_cnt[kx - 1u] = have;
       f_info[kx - 1u] = t_info[tid];
     }
-    nf = ktot;
-    emitted += ltot;
+    nf = tot & 0xffffu;
+    emitted += tot >> 16;
     __syncthreads();
   }
   // the leaf slots, with their random streams in slot order
@@ -629,7 +713,6 @@ __global__ void __launch_bounds__(T, 1024 / T)
 __device__ __forceinline__ void add_up(const Pool &p, const Table &t, bool on, int32_t s, int32_t leaf,
                                        uint32_t leaf_turn, uint32_t visits, uint32_t s1, uint32_t s2, uint32_t ppl,
                                        uint32_t *status) {
-  constexpr uint32_t kFull = 0xffffffffu;
   const int32_t root = on ? t.root[s] : -1;
   bool first = (leaf_turn & 1u) != 0;  // PLAYER_1 moved into the leaf
   int32_t n = leaf;
@@ -643,9 +726,8 @@ __device__ __forceinline__ void add_up(const Pool &p, const Table &t, bool on, i
     }
   }
   const uint32_t score = on ? (first ? s1 : s2) : 0u;
-  int same = 0;
-  __match_all_sync(kFull, on ? s : -1 - (int32_t)(threadIdx.x & 31u), &same);
-  if (same) {  // all on, one search
+  const int32_t s0 = __shfl_sync(kFull, s, 0);  // every lane takes part, also those without a leaf
+  if (__all_sync(kFull, on && s == s0)) {
     const uint32_t sum = __reduce_add_sync(kFull, score);
     if ((threadIdx.x & 31u) == 0) {
       atomicAdd(&p.info[root].z, 32u * visits);

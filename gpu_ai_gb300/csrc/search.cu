@@ -1009,7 +1009,12 @@ int enqueue_step(gpuai_searches *s, uint32_t q) {
                                          s->ctl + 1);
   };
   if (s->net) {
-    if (q <= 256) sel(select_kernel<true, 256>, 256);
+    // 16 warps, a node each, while two blocks per SM hold all searches: 1 to 4 %
+    // of a step (1 search x 64 leaves 120.6 -> 117.0 us, 200 x 64 194.8 -> 192.3,
+    // 300 x 256 461 -> 451); 16 leaves have no work for them (200 x 16: 136.5
+    // against 137.6 us)
+    const bool wide = q > 256 || (q > 16 && s->slots <= 2u * (uint32_t)s->sms);
+    if (!wide) sel(select_kernel<true, 256>, 256);
     else sel(select_kernel<true, 512>, 512);
   } else {
     if (q <= 128) sel(select_kernel<false, 128>, 128);

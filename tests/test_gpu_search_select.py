@@ -53,15 +53,15 @@ def test_nodes_with_few_and_many_children(lo, hi):
     _run(policy=0, ppl=2, q=100, budgets=[3000] * 4, caps=[20000] * 4, roots=roots, graph=True, steps=14)
 
 
-@pytest.mark.parametrize("lo,hi", [(2, 8), (9, 16), (17, 32), (33, 45)])
-def test_learned_splits_by_number_of_children(lo, hi):
+@pytest.mark.parametrize("lo,hi,q", [(2, 8, 43), (9, 16, 43), (17, 32, 43), (33, 45, 43), (9, 16, 15)])
+def test_learned_splits_by_number_of_children(lo, hi, q):
     """The slots of a learned node are handed out in fours, with the terms of up
     to 8, up to 16, up to 32 and more children laid out differently; 43 leaves
-    leave a remainder and a partly filled warp."""
+    leave a remainder and a partly filled warp, 15 take the narrower block."""
     from gpu_ai_gb300 import Net, Searches
     net = Net(0, max_batch=256, seed=1)
     net.set_params(_peaky_params(5))
-    gpu = Searches(3, 60000, 43, playouts_per_leaf=1, policy=0, seed=3)
+    gpu = Searches(3, 60000, q, playouts_per_leaf=1, policy=0, seed=3)
     gpu.set_net(net, value_weight=0.5, c_puct=1.5)
     learned = {"value_weight": 0.5, "c_puct": 1.5}
     o = S.SearchesOracle(3, 1, 0, 3, children=L.children, playouts=_replay, learned=learned)
@@ -70,10 +70,10 @@ def test_learned_splits_by_number_of_children(lo, hi):
         slots.append(gpu.add(r, 400, 15000, (i + 7) << 36))
         assert o.add(r, 400, 15000, (i + 7) << 36) == slots[-1]
     for step in range(10):
-        gpu.step(1, 43, True)
+        gpu.step(1, q, True)
         gpu.poll()
         lv = gpu.leaves(net=True)
-        o.step(43, net_value=lv["net_value"], net_logits=lv["net_logits"])
+        o.step(q, net_value=lv["net_value"], net_logits=lv["net_logits"])
         _compare_step(gpu, o, step, net=True)
         _compare_trees(gpu, o, slots, step, priors=True)
     gpu.close()

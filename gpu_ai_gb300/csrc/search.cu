@@ -61,7 +61,11 @@ namespace {
 
 constexpr uint32_t kExpanded = 1u, kTerminal = 2u, kEvaluated = 4u;  // node state bits (info.y >> 16)
 constexpr uint32_t kFull = 0xffffffffu;  // all lanes of a warp
-constexpr int kMaxSelectDepth = 512;
+// Levels a selection descends at most (tests compile a smaller limit in)
+#ifndef GPUAI_MAX_SELECT_DEPTH
+#define GPUAI_MAX_SELECT_DEPTH 512
+#endif
+constexpr int kMaxSelectDepth = GPUAI_MAX_SELECT_DEPTH;
 constexpr uint32_t kStatusSelectDepth = 8u;
 // Frontier entries whose expansions take nodes together in a step with Q leaves
 // per search (select_kernel).
@@ -687,10 +691,12 @@ __global__ void __launch_bounds__(T, 1024 / T)
     emitted += tot >> 16;
     __syncthreads();
   }
-  // the leaf slots, with their random streams in slot order
+  // the leaf slots, with their random streams in slot order; the slots of a
+  // selection that stopped at the depth limit play out the root, so that no
+  // kernel of the step meets an earlier step's entry (whose search may be gone)
   const unsigned long long sbase = t.stream_next[s];
-  if (tid < emitted && GA_IN_BOUNDS(off + tid < slots * lrn.max_leaves, status)) {
-    const int32_t n = s_leaf[tid];
+  if (tid < q && GA_IN_BOUNDS(off + tid < slots * lrn.max_leaves, status)) {
+    const int32_t n = tid < emitted ? s_leaf[tid] : root;
     l.board[off + tid] = p.board[n];
     l.node[off + tid] = n;
     l.search[off + tid] = (int32_t)s;
@@ -707,7 +713,8 @@ __global__ void __launch_bounds__(T, 1024 / T)
 // and, to a node that PLAYER_1 moved into, s1 half points, else s2 (the players
 // alternate along the path).  The root and the search's count take the same
 // addition from every leaf of the search: a warp whose leaves are all of one
-// search adds its sum there once.  (With an addition per leaf, and each node's
+// search adds its sum there once.  A path that does not end at the root adds
+// nothing there.  (With an addition per leaf, and each node's
 // board loaded for its mover, 16.5 against 8 us a step of 64 searches x 512
 // leaves.)
 __device__ __forceinline__ void add_up(const Pool &p, const Table &t, bool on, int32_t s, int32_t leaf,
@@ -725,9 +732,10 @@ __device__ __forceinline__ void add_up(const Pool &p, const Table &t, bool on, i
       n = p.parent[n];
     }
   }
+  const bool ends = on && n >= 0 && n == root;
   const uint32_t score = on ? (first ? s1 : s2) : 0u;
   const int32_t s0 = __shfl_sync(kFull, s, 0);  // every lane takes part, also those without a leaf
-  if (__all_sync(kFull, on && s == s0)) {
+  if (__all_sync(kFull, ends && s == s0)) {
     const uint32_t sum = __reduce_add_sync(kFull, score);
     if ((threadIdx.x & 31u) == 0) {
       atomicAdd(&p.info[root].z, 32u * visits);
@@ -735,8 +743,10 @@ __device__ __forceinline__ void add_up(const Pool &p, const Table &t, bool on, i
       atomicAdd(&t.done[s], 32ull * ppl);
     }
   } else if (on) {
-    atomicAdd(&p.info[root].z, visits);
-    atomicAdd(&p.info[root].w, score);
+    if (ends) {
+      atomicAdd(&p.info[root].z, visits);
+      atomicAdd(&p.info[root].w, score);
+    }
     atomicAdd(&t.done[s], (unsigned long long)ppl);
   }
 }

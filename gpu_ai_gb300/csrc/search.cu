@@ -830,7 +830,12 @@ __global__ void __launch_bounds__(kEvalThreads)
   const bool over = k == 0 || ((b.meta >> 8) & 0xffu) >= (uint32_t)kDrawPlies;
   if (on && gl == 0) l.value[i] = over ? kTerminalLeaf : dm::det_tanh(vraw[i]);
   const int32_t n = on ? l.node[i] : 0;
-  const bool fresh = on && !over && !((p.info[n].y >> 16) & (kEvaluated | kTerminal));
+  // One lane reads the node's state for its group: other groups with the same
+  // node set kEvaluated meanwhile, and the group's maximum and sum need all its
+  // lanes or none.  (A group that finds it set leaves the priors to the others,
+  // which write the whole list, the same one.)
+  const uint32_t state = __shfl_sync(kFull, on && gl == 0 ? p.info[n].y >> 16 : 0u, lane0);
+  const bool fresh = on && !over && !(state & (kEvaluated | kTerminal));
   const __nv_bfloat16 *lr = logits + (size_t)i * net::kOut;
   const bool shared = fresh && simple && k <= (int)kPriors;
   if (__any_sync(kFull, shared)) {

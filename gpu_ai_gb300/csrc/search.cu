@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(kEvalThreads)
         p.prior[(size_t)n * kPriors + gl + G * j] = __float2half_rn(dm::div(x[j], sum));
   }
   if (!fresh || gl != 0) return;
-  if (!simple && k <= (int)kPriors) {
+  if (!simple && k >= 1 && k <= (int)kPriors) {  // (k is -1 where a capture passes the depth limit)
     uint16_t pair[kPriors] = {};
     uint8_t of[kPriors];
     uint8_t mult[kPriors];

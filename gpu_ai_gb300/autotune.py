@@ -8,7 +8,10 @@ playouts and
 (2) the batched-search step's leaves per search and playouts per leaf, and
 caches the fastest settings in a JSON file keyed by GPU name (default
 ``~/.cache/gpu_ai_gb300/autotune.json``).  ``apply(engine)`` sets a cached
-layout and launch shape on an Engine.
+layout and launch shape on an Engine.  An entry that is the Engine's own default
+leaves the choice by batch size on (gpuai_set_launch); any other holds for
+batches of every size, the small ones too, although it was measured on a large
+one.
 
     python -m gpu_ai_gb300.autotune [--quick] [--cache PATH]
 """

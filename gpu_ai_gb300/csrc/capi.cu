@@ -98,19 +98,22 @@ namespace ga {
 int record_error(int code, const char *msg) { return fail(code, "%s", msg); }
 }  // namespace ga
 
+constexpr int kDefaultBlock[3] = {2 * ga::kPlayoutBlock, ga::kPlayoutBlock, ga::kPlayoutBlock};
+
 struct gpuai_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   int sms = 0;
-  // threads per block by policy (launch_shape takes others for small batches): the uniform random kernel runs 512-thread blocks (2 per SM; ~1 % faster
-  // than 4 x 256 on 64 x 4,096 batches, equal on large ones: a block packs its games over 16 warps when
-  // the work runs out); the 80-register reference-heuristic kernel fits 3 x 256 per SM
-  int block[3] = {2 * ga::kPlayoutBlock, ga::kPlayoutBlock, ga::kPlayoutBlock};
+  // threads per block by policy (launch_shape takes others for small batches): the uniform random kernel
+  // runs 512-thread blocks (2 per SM; ~1 % faster than 4 x 256 on 64 x 4,096 batches, equal on large ones:
+  // a block packs its games over 16 warps when the work runs out); the 80-register reference-heuristic
+  // kernel fits 3 x 256 per SM
+  int block[3] = {kDefaultBlock[0], kDefaultBlock[1], kDefaultBlock[2]};
   int blocks_per_sm[3] = {0, 0, 0};  // resident blocks per SM used for the grid
+  int default_blocks_per_sm[3] = {0, 0, 0};
   int max_blocks_per_sm[3] = {0, 0, 0};
   int layout[3] = {ga::kLayoutThread, ga::kLayoutThread, ga::kLayoutThread};
-  bool chosen[3] = {false, false, false};  // launch shape or layout set by the caller
-  int small_blocks_per_sm[3][2] = {};      // resident blocks of 128 and 256 threads (0: not asked yet)
+  int small_blocks_per_sm[3][2] = {};  // resident blocks of 128 and 256 threads (0: not asked yet)
   Control *ctl = nullptr;  // device
   Control last_host{};      // control block of the last host-buffer call, as read back
   bool last_was_host = false;
@@ -136,8 +139,9 @@ int set_device(gpuai_ctx *ctx) {
   return GPUAI_OK;
 }
 
-// Launch shape of `total` playouts: the caller's, or by size.  A batch that fits
-// the GPU's lanes has no steady state, in which the uniform random policy's wide
+// Launch shape of `total` playouts: the one that is set, or, while that is the
+// default one (never changed, or set back), by size.  A batch that fits the
+// GPU's lanes has no steady state, in which the uniform random policy's wide
 // blocks pay (262,144 playouts: 315 us with 512 threads, 325 with 256), and its
 // blocks' barriers and packing cost less with fewer warps: 140,000 playouts
 // 194 us with 256 threads, 209 with 512; 16,000 150 against 156; with a handful
@@ -147,8 +151,9 @@ int set_device(gpuai_ctx *ctx) {
 int launch_shape(gpuai_ctx *ctx, int policy, uint32_t total, int *block, int *grid) {
   *block = ctx->block[policy];
   int per_sm = ctx->blocks_per_sm[policy];
-  if (!ctx->chosen[policy]) {
-    const uint32_t lanes = (uint32_t)ctx->sms * (uint32_t)(ctx->blocks_per_sm[policy] * ctx->block[policy]);
+  if (ctx->layout[policy] == ga::kLayoutThread && *block == kDefaultBlock[policy] &&
+      per_sm == ctx->default_blocks_per_sm[policy]) {
+    const uint32_t lanes = (uint32_t)ctx->sms * (uint32_t)(per_sm * *block);
     const int which = total <= 8u * (uint32_t)ctx->sms ? 0 : (total <= lanes ? 1 : 2);
     if (which < 2) {
       *block = which == 0 ? 128 : 256;
@@ -218,7 +223,7 @@ int gpuai_create(int device, gpuai_ctx **out) {
     e = ga::playout_occupancy(p, ctx->block[p], &ctx->max_blocks_per_sm[p]);
     if (e != cudaSuccess) rc = cuda_fail(e, "occupancy query");
     else if (ctx->max_blocks_per_sm[p] < 1) ctx->max_blocks_per_sm[p] = 1;
-    ctx->blocks_per_sm[p] = ctx->max_blocks_per_sm[p];
+    ctx->blocks_per_sm[p] = ctx->default_blocks_per_sm[p] = ctx->max_blocks_per_sm[p];
   }
   if (rc == GPUAI_OK) {
     e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
@@ -268,7 +273,6 @@ int gpuai_set_launch(gpuai_ctx *ctx, int32_t policy, int32_t block_threads, int3
   CK(ga::playout_occupancy(policy, block_threads, &maxb, ctx->layout[policy]), "occupancy query");
   if (maxb < 1) return fail(GPUAI_ERR_INVALID, "gpuai_set_launch: block of %d threads cannot be resident", block_threads);
   if (blocks_per_sm < 0) return fail(GPUAI_ERR_INVALID, "gpuai_set_launch: negative blocks_per_sm");
-  ctx->chosen[policy] = true;
   ctx->block[policy] = block_threads;
   ctx->max_blocks_per_sm[policy] = maxb;
   ctx->blocks_per_sm[policy] = (blocks_per_sm == 0 || blocks_per_sm > maxb) ? maxb : blocks_per_sm;
@@ -288,7 +292,6 @@ int gpuai_set_layout(gpuai_ctx *ctx, int32_t policy, int32_t layout) {
   int maxb = 0;
   CK(ga::playout_occupancy(policy, ctx->block[policy], &maxb, layout), "occupancy query");
   if (maxb < 1) return fail(GPUAI_ERR_INVALID, "gpuai_set_layout: the kernel cannot be resident");
-  ctx->chosen[policy] = true;
   ctx->layout[policy] = layout;
   ctx->max_blocks_per_sm[policy] = maxb;
   ctx->blocks_per_sm[policy] = maxb;

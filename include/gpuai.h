@@ -119,9 +119,10 @@ int gpuai_device_info(gpuai_ctx *ctx, int32_t *sms, int32_t *blocks_per_sm, int3
 /* Launch shape of the playout kernel for `policy`: threads per block (64,
  * 128, 256 or 512) and resident blocks per SM the persistent grid uses
  * (0 = as many as fit).  The grid is SMs x blocks_per_sm, or fewer blocks for
- * small batches.  Until a shape or layout is set, batches that fit the GPU's
- * lanes run in smaller blocks than the default shape that gpuai_get_launch
- * reports.  Results do not depend on the launch shape.  This is the
+ * small batches.  With the shape and layout of a new context, never changed or
+ * set back, batches that fit the GPU's lanes run in smaller blocks than the
+ * shape that gpuai_get_launch reports; any other shape holds for every batch.
+ * Results do not depend on the launch shape.  This is the
  * knob the autotuner sweeps; it has no counterpart in the reference, whose
  * drivers hard-code <<<N,32>>>, <<<N/128,128>>> and the coarse grid
  * (src/multiplePlayout.cu:77, src/singlePlayout.cu:86-99, src/coarsePlayout.cu:113-115). */

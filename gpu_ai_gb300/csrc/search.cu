@@ -864,10 +864,11 @@ __global__ void __launch_bounds__(kEvalThreads)
     }
 #pragma unroll
     for (int j = 0; j < J; j++)
-      if (shared && gl + G * j < k)
-        p.prior[(size_t)n * kPriors + gl + G * j] = __float2half_rn(dm::div(x[j], sum));
+      if (shared)
+        p.prior[(size_t)n * kPriors + gl + G * j] = __float2half_rn(gl + G * j < k ? dm::div(x[j], sum) : 0.0f);
   }
   if (!fresh || gl != 0) return;
+  int written = shared ? (int)kPriors : 0;  // the rest of the node's priors are zero
   if (!simple && k >= 1 && k <= (int)kPriors) {  // (k is -1 where a capture passes the depth limit)
     uint16_t pair[kPriors] = {};
     uint8_t of[kPriors];
@@ -901,7 +902,9 @@ __global__ void __launch_bounds__(kEvalThreads)
       const int u = of[j];
       p.prior[(size_t)n * kPriors + j] = __float2half_rn(dm::div(dm::div(e[u], sum), (float)mult[u]));
     }
+    written = k;
   }
+  for (int j = written; j < (int)kPriors; j++) p.prior[(size_t)n * kPriors + j] = __float2half_rn(0.0f);
   atomicOr(&p.info[n].y, kEvaluated << 16);
 }
 
@@ -1447,6 +1450,8 @@ int gpuai_searches_nodes(gpuai_searches *s, int32_t slot, uint32_t max_nodes, ui
       info[4 * i + 3] = inf[i].w;
     }
     if (parent) parent[i] = par[i] < 0 ? -1 : par[i] - r;
+    // a node that was not evaluated has no priors (the range may have been another search's)
+    if (priors && !((inf[i].y >> 16) & kEvaluated)) std::memset(priors + (size_t)i * kPriors, 0, 2 * kPriors);
   }
   return GPUAI_OK;
 }

@@ -195,7 +195,8 @@ int gpuai_searches_set_proposal(gpuai_searches *s, uint32_t guided_plies, float 
  * 4 evaluated by the network), playouts through the node (visit units for
  * learned searches), score in half points of the player who moved into the
  * node.  boards, parent (-1 for the root) and priors (32 FP16 bit patterns
- * per node, learned searches only) are optional too. */
+ * per node, learned searches only; zero past the node's moves and for a node
+ * that is not evaluated or has more than 32) are optional too. */
 int gpuai_searches_nodes(gpuai_searches *s, int32_t slot, uint32_t max_nodes, uint32_t *info, gpuai_board *boards,
                          int32_t *parent, uint16_t *priors, uint32_t *nnodes);
 /* The last step's leaf slots, in slot order (searches in slot order, each

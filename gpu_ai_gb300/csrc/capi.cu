@@ -142,12 +142,16 @@ int set_device(gpuai_ctx *ctx) {
 // Launch shape of `total` playouts: the one that is set, or, while that is the
 // default one (never changed, or set back), by size.  A batch that fits the
 // GPU's lanes has no steady state, in which the uniform random policy's wide
-// blocks pay (262,144 playouts: 315 us with 512 threads, 325 with 256), and its
-// blocks' barriers and packing cost less with fewer warps: 140,000 playouts
-// 194 us with 256 threads, 209 with 512; 16,000 150 against 156; with a handful
-// of games per SM 128 threads are better still (1000 playouts of one each 112,
-// 117 with 256 or 512; eps-greedy 149, 153, 160).  The grid is a block per
-// playout up to the resident ones (the kernel deals a small batch out over them).
+// blocks pay, and its blocks' barriers and packing cost less with fewer warps.
+// Host calls on positions 0-30 plies deep with 128 / 256 / 512 threads (256 for
+// the other policies' default), medians in us on one box, two runs within 1 %:
+//   256 playouts of one position 107 / 108 / 115; 1000 positions once 121 / 120 /
+//   129, eps-greedy 166 / 169; 64 x 250 144 / 152 / 158; 70 x 2000 238 / 239 / 242;
+//   64 x 4,096 318 / 328 / 322; eps-greedy 16,384 x 4 360 / 371; heuristic
+//   64 x 500 348 / 354.
+// (Between the two limits 128 threads were up to 5 % below 256 there: the first
+// limit could lie higher.)  The grid is a block per playout up to the resident
+// ones (the kernel deals a small batch out over them).
 int launch_shape(gpuai_ctx *ctx, int policy, uint32_t total, int *block, int *grid) {
   *block = ctx->block[policy];
   int per_sm = ctx->blocks_per_sm[policy];

@@ -82,8 +82,8 @@ __device__ __forceinline__ uint32_t vload(const uint32_t *p) { return *reinterpr
 
 // The random draws of a game whose ring of eight buffered draws is a column of
 // shared memory: draw k is word k % 8 of the column (consecutive threads,
-// consecutive banks), read with one load where DrawRing selects among eight
-// registers.  refill() keeps at least four draws buffered.
+// consecutive banks), one load at a changing index (eight registers would need
+// a select among them).  refill() keeps at least four draws buffered.
 template <uint32_t TAG>
 struct SharedRing {
   uint32_t *ring;   // word 0 of column 0
@@ -186,8 +186,8 @@ struct HeurGame {  // reference heuristic: two draws per move, generated where t
 template <int POLICY, bool POSITIONS> struct GameOf { using type = RotGame<POSITIONS ? 1u : 0u>; };
 template <> struct GameOf<1, false> { using type = HeurGame; };
 
-// Bound by the integer (ALU) pipe while every lane has a game (82 % of its
-// peak on 20,011 positions with 4.0 M playouts, 58 % of the lanes active: the
+// Bound by the integer (ALU) pipe while every lane has a game (84 % of its
+// peak on 20,011 positions with 4.0 M playouts, 65 % of the lanes active: the
 // rest is the code of the multi-jump plies, which few lanes of a warp run at a
 // time), and by the length of the last games once the work runs out.  Plies on
 // rotated bitboards from the side to move instead of rules.cuh's, draws in
@@ -368,8 +368,8 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
     // at the start, each block's share over as few warps as hold it: the host
     // launches a block per playout up to the resident ones, so a small batch has
     // few games per SM and per warp, each at a lone game's latency (256 playouts
-    // of one position, host call: 153 -> 126 us; 65,536 eps-greedy ones: 355 ->
-    // 337 us).  More warps with fewer games each, here or after packing, are
+    // of one position, host call: 146-153 -> 116-126 us on two boxes; 65,536
+    // eps-greedy ones: 355 -> 337 us).  More warps with fewer games each, here or after packing, are
     // slower once an SM holds more than a few (2, 4, 8 warps per block at least:
     // 1-5 % on the benchmark batch, 3-39 % on 65,536 playouts).
     const uint32_t share = POSITIONS ? a.total : (a.total + gridDim.x - 1u) / gridDim.x;

@@ -1028,9 +1028,9 @@ cudaError_t gemm(const CUtensorMap &a, const CUtensorMap &b, uint32_t m_rows, ui
   g.tmem_cols = bn <= 64 ? 64u : (bn <= 128 ? 128u : 256u);
   g.kb_per_split = kb_total / splits;
   const uint32_t stage_bytes = kABytes + bn * 128u;
-  // A product of the training step's critical chain (the launches with
-  // `pdl`) whose grid is at most one CTA per SM gets twice the ring: more
-  // loads in flight.  The side streams' products keep room for a second CTA
+  // A product of a chain (the launches with `pdl`: the training step's critical
+  // one, and inference) whose grid is at most one CTA per SM gets twice the
+  // ring: more loads in flight.  The side streams' products keep room for a second CTA
   // on each SM, where they run beside the chain.
   const uint32_t ctas = (m_rows / kBM) * (n_total / bn) * splits;
   const uint32_t budget = pdl && ctas <= sm_count() ? 2u * kRingBudget : kRingBudget;
@@ -1108,8 +1108,10 @@ namespace {
 // The products launch early (programmatic dependent launch) but for calls whose
 // row count is on the device, which their kernels read first.  These chains are
 // launch latency up to a few thousand boards: with the tanh in the last epilogue
-// instead of a kernel of its own, a call takes 59 instead of 71 us for 1 board,
-// 148 instead of 161 for 1000, 425 instead of 436 for 4000.
+// instead of a kernel of its own, a repeated call takes 56-58 instead of 68-71 us
+// for 1 board, 146-150 instead of 158-162 for 1000, 421-432 instead of 430-438
+// for 4000 (four interleaved runs on one box; 156 instead of 168 for 1000 boards
+// that change from call to call).
 cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards, uint32_t n, const uint32_t *dev_n,
                          uint32_t rows, uint32_t *status, bool train, cudaStream_t s, float *value = nullptr) {
   const bool pdl = dev_n == nullptr;

@@ -806,8 +806,11 @@ constexpr uint32_t kKingPeriod = 16, kKingPhase = 6;
 GA_HD constexpr uint32_t king_period(int policy) { return policy == 0 ? kKingPeriod : kKingPeriod / 2; }
 // Men's multi-jumps are deferred for the eps-greedy and reference-heuristic
 // policies only: the uniform random policy plays them at once (measured on
-// one box: 0.3748 against 0.3761 ms on the benchmark batch, 3.92 against
-// 3.96 ms on 64 x 65,536), the eps-greedy one loses 3 % without deferral.
+// this file's plies, on one box: 0.3748 against 0.3761 ms on the benchmark
+// batch, 3.92 against 3.96 ms on 64 x 65,536; the eps-greedy one loses 3 %
+// without deferral.  On rot.cuh's plies the reference heuristic takes 904
+// instead of 849 us without it, and a deferral of 2 or 4 is equal or slower
+// for the uniform policy).
 GA_HD constexpr bool defer_men(int policy) { return policy != 0; }
 // a deferred ply must have a phase that comes round, or its game never ends
 static_assert((kMenPeriod & (kMenPeriod - 1u)) == 0 && kMenPhase < kMenPeriod, "men's phase outside its period");
@@ -875,9 +878,13 @@ GA_HD int play_ply_fast(Board &b, Pick &&pick) {
   return play_ply_sched(b, pick, true, true);
 }
 
-// Random draws of one stream buffered eight at a time, so that a warp can
+// Random draws of one stream buffered eight at a time, so that a warp could
 // generate Philox blocks for all its lanes at the same loop iteration.
-// refill() keeps at least four draws buffered; next() consumes one.
+// refill() keeps at least four draws buffered; next() consumes one.  The
+// kernels buffer theirs in shared memory (SharedRing of kernels.cu, the same
+// schedule); this ring, RingOnDemand, play_ply_eps_sched and
+// play_ply_heur_sched below are the CPU tests' references on this file's
+// squares for the plies of rot.cuh.
 struct DrawRing {
   uint32_t a0, a1, a2, a3, b0, b1, b2, b3;  // slots 0-3 and 4-7
   uint32_t k, avail;
@@ -1013,6 +1020,7 @@ GA_HD int ply_eps_greedy(Board &b, Rng &rs) {
 }
 
 // ------------------------------------------------------------ eps-greedy without enumeration
+// (a reference of the CPU tests; the kernels play rot.cuh's)
 
 // Bit plane q of a per-square value c + sgn * row (4 squares per row).
 GA_HD constexpr uint32_t row_value_plane(int q, int c, int sgn) {
@@ -1145,6 +1153,7 @@ GA_HD int play_ply_eps_sched(Board &b, Rng &rs, bool men_now, bool king_now) {
 }
 
 // ------------------------------------------------------------ reference heuristic, one step per move
+// (a reference of the CPU tests; the kernels play rot.cuh's)
 
 // The reference-heuristic ply (the move and the draws of ply_ref_heuristic)
 // for plies where no capture can continue: the ply's four material weights are

@@ -1039,6 +1039,11 @@ int enqueue_step(gpuai_searches *s, uint32_t q) {
     else if (q <= 256) sel(select_kernel<false, 256>, 256);
     else sel(select_kernel<false, 512>, 512);
   }
+  // The playouts' number is known on the device alone when a step is enqueued
+  // (and a captured step is replayed as the searches finish), so every step
+  // launches 256-thread blocks: us a step with 256 / 128 threads, one search of 64
+  // leaves x 2 93.6 / 91.8, 4 searches 114 / 106, 16 of 64 x 8 132 / 131, 64 of
+  // 128 x 8 185 / 187.
   PlayoutArgs a;
   a.pos = reinterpret_cast<const Board *>(s->leaves.board);
   a.offsets = nullptr;

@@ -144,7 +144,7 @@ int set_device(gpuai_ctx *ctx) {
 // GPU's lanes has no steady state, in which the uniform random policy's wide
 // blocks pay, and its blocks' barriers and packing cost less with fewer warps.
 // Host calls on positions 0-30 plies deep with 128 / 256 / 512 threads (256 for
-// the other policies' default), medians in us on one box, two runs within 1 %:
+// the other policies' default), medians in us on one GPU, two runs within 1 %:
 //   256 playouts of one position 107 / 108 / 115; 1000 positions once 121 / 120 /
 //   129, eps-greedy 166 / 169; 64 x 250 144 / 152 / 158; 70 x 2000 238 / 239 / 242;
 //   64 x 4,096 318 / 328 / 322; eps-greedy 16,384 x 4 360 / 371; heuristic

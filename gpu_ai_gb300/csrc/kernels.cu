@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(BLOCK, (playout_min_blocks<POLICY, BLOCK>()))
     // at the start, each block's share over as few warps as hold it: the host
     // launches a block per playout up to the resident ones, so a small batch has
     // few games per SM and per warp, each at a lone game's latency (256 playouts
-    // of one position, host call: 146-153 -> 116-126 us on two boxes; 65,536
+    // of one position, host call: 146-153 -> 116-126 us on two GPUs; 65,536
     // eps-greedy ones: 355 -> 337 us).  More warps with fewer games each, here or after packing, are
     // slower once an SM holds more than a few (2, 4, 8 warps per block at least:
     // 1-5 % on the benchmark batch, 3-39 % on 65,536 playouts).

@@ -1110,7 +1110,7 @@ namespace {
 // launch latency up to a few thousand boards: with the tanh in the last epilogue
 // instead of a kernel of its own, a repeated call takes 56-58 instead of 68-71 us
 // for 1 board, 146-150 instead of 158-162 for 1000, 421-432 instead of 430-438
-// for 4000 (four interleaved runs on one box; 156 instead of 168 for 1000 boards
+// for 4000 (four interleaved runs on one GPU; 156 instead of 168 for 1000 boards
 // that change from call to call).
 cudaError_t forward_impl(const gpuai_net *net, Fwd &w, const gpuai_board *boards, uint32_t n, const uint32_t *dev_n,
                          uint32_t rows, uint32_t *status, bool train, cudaStream_t s, float *value = nullptr) {

@@ -806,7 +806,7 @@ constexpr uint32_t kKingPeriod = 16, kKingPhase = 6;
 GA_HD constexpr uint32_t king_period(int policy) { return policy == 0 ? kKingPeriod : kKingPeriod / 2; }
 // Men's multi-jumps are deferred for the eps-greedy and reference-heuristic
 // policies only: the uniform random policy plays them at once (measured on
-// this file's plies, on one box: 0.3748 against 0.3761 ms on the benchmark
+// this file's plies, on one GPU: 0.3748 against 0.3761 ms on the benchmark
 // batch, 3.92 against 3.96 ms on 64 x 65,536; the eps-greedy one loses 3 %
 // without deferral.  On rot.cuh's plies the reference heuristic takes 904
 // instead of 849 us without it, and a deferral of 2 or 4 is equal or slower
